@@ -18,7 +18,7 @@
 #include <tuple>
 #include <vector>
 
-#include "kernels.cuh"
+#include "group.cuh"
 
 namespace pgeof {
 
@@ -73,35 +73,47 @@ __global__ void box_init_kernel(uint32_t* box, int n_clouds) {
         box[i] = (i % 6) < 3 ? 0xffffffffu : 0u;
 }
 
+// Cells of one cloud for edge h (x edge h / xsub): their number per axis in d
+// and in all, or 0 when they pass `cap`.
+__device__ uint64_t cloud_cells(const float* mn, const float* mx, double h, int xsub, uint64_t cap, int (&d)[3]) {
+    uint64_t G = 1;
+    for (int a = 0; a < 3; ++a) {
+        const double cells = floor(((double)mx[a] - (double)mn[a]) / (a == 0 ? h / xsub : h)) + 1.0;
+        if (cells > 2.0e9) return 0;
+        d[a] = (int)cells;
+        G *= (uint64_t)d[a];
+        if (G > cap) return 0;
+    }
+    return G;
+}
+
 // Grid parameters of one cloud for edge h, growing h until the cloud's cell cap
-// holds (same rules as the single-cloud build).
-__device__ void cloud_params(const float* mn, const float* mx, double h, uint64_t cap, GridParams& g) {
+// holds (same rules as the single-cloud build); x_split: cells cut along x as
+// far as the cap allows (see GridParams).
+__device__ void cloud_params(const float* mn, const float* mx, double h, uint64_t cap, bool x_split, GridParams& g) {
     for (int it = 0; it < 200; ++it) {
-        uint64_t G = 1;
         int d[3];
-        bool ok = true;
-        for (int a = 0; a < 3; ++a) {
-            const double cells = floor(((double)mx[a] - (double)mn[a]) / h) + 1.0;
-            if (cells > 2.0e9) {
-                ok = false;
-                break;
+        uint64_t G = cloud_cells(mn, mx, h, 1, cap, d);
+        if (G) {
+            int xs = 1;
+            for (int t = 4; x_split && t > 1; t /= 2) {
+                int e[3];
+                const uint64_t fine = cloud_cells(mn, mx, h, t, cap, e);
+                if (fine) {
+                    G = fine;
+                    xs = t;
+                    for (int a = 0; a < 3; ++a) d[a] = e[a];
+                    break;
+                }
             }
-            d[a] = (int)cells;
-            G *= (uint64_t)d[a];
-            if (G > cap) {
-                ok = false;
-                break;
-            }
-        }
-        if (ok) {
             g.ox = mn[0];
             g.oy = mn[1];
             g.oz = mn[2];
             g.h = (float)h;
             g.inv_h = (float)(1.0 / h);
-            g.hx = g.h;
-            g.inv_hx = g.inv_h;
-            g.xsub = 1;
+            g.hx = (float)(h / xs);
+            g.inv_hx = (float)(1.0 / (h / xs));
+            g.xsub = xs;
             g.gx = d[0];
             g.gy = d[1];
             g.gz = d[2];
@@ -141,7 +153,7 @@ __global__ void batch_params_kernel(const uint32_t* __restrict__ box, const uint
             if (m_w > 0.0) h = fmax(h * fmin(16.0, fmax(1.0 / 16.0, sqrt(target / m_w))), floor_h);
         }
         GridParams gp;
-        cloud_params(mn, mx, h, cap, gp);
+        cloud_params(mn, mx, h, cap, pass == 1, gp);
         g[c] = gp;
     }
     __syncthreads();
@@ -270,7 +282,7 @@ size_t layout(BatchWorkspace& w, char* base) {
     w.pts = (SPoint<float>*)take(n * sizeof(SPoint<float>));
     w.xyz4 = (float4*)take(n * sizeof(float4));
     w.nn_ptr = (uint32_t*)take((n + 1) * 4);
-    w.words = (uint32_t*)take((n + 8) * 4);
+    w.words = (uint32_t*)take(search_batch_words(n) * 4);
     w.scan_part = (uint32_t*)take((cells / 1024 + 2) * 4);
     w.defer = (unsigned long long*)take((n + 1) * 8);
     return o;
@@ -320,7 +332,9 @@ int run_pipeline(BatchWorkspace& w, const float* xyz, uint32_t* idx, float* d2, 
     PGEOF_TRY(current_device_info(&di));
     const int nc = w.n_clouds;
     const uint64_t n = w.n;
-    const float target = std::min(48.0f, std::max(2.0f, (float)w.k / 3.5f * tune.cell));
+    const bool grouped = use_groups(w.n, w.n, w.k);
+    const float target = grouped ? (float)group_occupancy(w.k) * tune.cell
+                                 : std::min(48.0f, std::max(2.0f, (float)w.k / 3.5f * tune.cell));
     // 1. bounding boxes
     box_init_kernel<<<blocks_for(6 * (uint64_t)nc, 256, di->sm_count), 256, 0, s>>>(w.box, nc);
     {
@@ -357,7 +371,7 @@ int run_pipeline(BatchWorkspace& w, const float* xyz, uint32_t* idx, float* d2, 
     ct.cell_base = w.cell_base;
     ct.off = w.off;
     ct.n = nc;
-    PGEOF_TRY(launch_search_batch(ct, w.cell_start, w.pts, n, w.k, idx, d2, w.words, w.words + 8, s, tune.chunk));
+    PGEOF_TRY(launch_search_batch(ct, w.cell_start, w.pts, n, w.k, idx, d2, w.words, s, grouped ? target : 0.0f, tune.chunk));
     // 5. features from the kNN rows (CSR with nn_ptr = k * row)
     if (features) {
         PGEOF_TRY(pad_xyz(xyz, n, w.xyz4, s));

@@ -19,7 +19,7 @@
 #include <cstring>
 #include <mutex>
 
-#include "kernels.cuh"
+#include "group.cuh"
 
 namespace pgeof {
 
@@ -227,10 +227,11 @@ struct HostBox {
 struct EdgeKey {
     uint64_t n;
     uint32_t k;
+    bool grouped;
     float h_min, h_max;
     float box[6];
     bool operator==(const EdgeKey& o) const {
-        return n == o.n && k == o.k && h_min == o.h_min && h_max == o.h_max && memcmp(box, o.box, sizeof(box)) == 0;
+        return n == o.n && k == o.k && grouped == o.grouped && h_min == o.h_min && h_max == o.h_max && memcmp(box, o.box, sizeof(box)) == 0;
     }
 };
 std::mutex g_edge_mu;
@@ -333,7 +334,7 @@ int exclusive_scan_into(const uint32_t* in, uint32_t G, uint32_t* out, uint32_t*
 
 template <typename T>
 int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h_max, GridIndex<T>& out,
-               cudaStream_t s) {
+               cudaStream_t s, bool grouped) {
     out.n = n;
     if (n == 0) return PGEOF_OK;
     if (n >= 0xffffffffull) return fail(PGEOF_ERR_INVALID_ARGUMENT, "point clouds are limited to 2^32-1 points");
@@ -369,7 +370,8 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
     // k / 12 is 19% faster at k = 50 than k / 3.5, on an outdoor scene of
     // walls and ground k / 3.5 is best. The dimension comes from two trial
     // histograms: (occupancy - 1) scales as h^dim (the 1 is the point itself).
-    const double target2 = std::min(48.0, std::max(2.0, (double)k_target / 3.5));
+    out.grouped = grouped ? (float)group_occupancy(k_target) : 0.0f;
+    const double target2 = grouped ? group_occupancy(k_target) : std::min(48.0, std::max(2.0, (double)k_target / 3.5));
     const uint64_t cap = std::max<uint64_t>(4 * n, 1u << 16);
     const double hmin = h_min > 0 ? (double)h_min : 0.0;
     const double hmax = h_max > 0 ? (double)h_max : 1e300;
@@ -383,7 +385,7 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
     };
     double h0 = clamp_h(std::cbrt(vol * target2 / (double)n));
     double h = h0;
-    EdgeKey key{n, k_target, h_min, h_max, {b.mn[0], b.mn[1], b.mn[2], b.mx[0], b.mx[1], b.mx[2]}};
+    EdgeKey key{n, k_target, grouped, h_min, h_max, {b.mn[0], b.mn[1], b.mn[2], b.mx[0], b.mx[1], b.mx[2]}};
     double cached = 0.0;
     if (edge_cache_get(key, cached)) {
         h = cached;
@@ -419,7 +421,7 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
             }
         }
         // volume-filling clouds: finer cells, placed by (m - 1) ~ h^dim
-        if (m0 > 1.05 && m1 > 1.05 && h1 != h0) {
+        if (!grouped && m0 > 1.05 && m1 > 1.05 && h1 != h0) {
             double dim = std::log((m0 - 1.0) / (m1 - 1.0)) / std::log(h0 / h1);
             if (!std::isfinite(dim)) dim = 2.0;
             dim = std::min(3.0, std::max(1.0, dim));
@@ -504,8 +506,8 @@ int sort_queries(const T* q, uint64_t m, const GridParams& g, Scratch& out_mem, 
     return check_launch("scatter_kernel(queries)");
 }
 
-template int build_grid<float>(const float*, uint64_t, uint32_t, float, float, GridIndex<float>&, cudaStream_t);
-template int build_grid<double>(const double*, uint64_t, uint32_t, float, float, GridIndex<double>&, cudaStream_t);
+template int build_grid<float>(const float*, uint64_t, uint32_t, float, float, GridIndex<float>&, cudaStream_t, bool);
+template int build_grid<double>(const double*, uint64_t, uint32_t, float, float, GridIndex<double>&, cudaStream_t, bool);
 template int sort_queries<float>(const float*, uint64_t, const GridParams&, Scratch&, SPoint<float>**, Scratch&,
                                  cudaStream_t);
 template int sort_queries<double>(const double*, uint64_t, const GridParams&, Scratch&, SPoint<double>**, Scratch&,

@@ -15,7 +15,7 @@
 #include <utility>
 #include <vector>
 
-#include "kernels.cuh"
+#include "group.cuh"
 
 namespace pgeof {
 namespace {
@@ -133,7 +133,8 @@ int pgeof_index_create_f32(const float* data, int64_t n_data, uint32_t k_hint, f
     // the cell-size rule of the per-call entry points: kNN steers the occupancy
     // towards k, a radius clamps the edge to [r/4, r]
     if (st == PGEOF_OK)
-        st = build_grid<float>(data, ix->n, ix->k_hint, radius_hint / 4.0f, radius_hint, ix->grid, s);
+        st = build_grid<float>(data, ix->n, ix->k_hint, radius_hint / 4.0f, radius_hint, ix->grid, s,
+                               use_groups(ix->n, ix->n, ix->k_hint));
     if (st == PGEOF_OK) st = ix->xyz4.alloc(ix->n * sizeof(float4), s);
     if (st == PGEOF_OK) {
         const int blocks = (int)std::min<uint64_t>((ix->n + 255) / 256, 4096);

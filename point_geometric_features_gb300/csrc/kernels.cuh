@@ -107,14 +107,16 @@ struct GridIndex {
     uint32_t* cell_start = nullptr;  // n_cells + 1 (device)
     SPoint<T>* pts = nullptr;        // n (device), cell order
     Scratch cell_mem, pts_mem;
+    float grouped = 0.0f;  // > 0: cells sized for the grouped search, with this occupancy
 };
 
 // Build the index of `xyz` (device, row-major (n, 3)). `k_target` steers the
 // cell size towards ~k_target/3.5 points per cell around an average point;
-// `h_min`/`h_max` (> 0) clamp the edge (radius searches).
+// `h_min`/`h_max` (> 0) clamp the edge (radius searches). `grouped`: cells for
+// the grouped search.
 template <typename T>
 int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h_max, GridIndex<T>& out,
-               cudaStream_t s);
+               cudaStream_t s, bool grouped = false);
 
 // Counting-sort arbitrary query points into `grid`'s cell order; `start`
 // receives the per-cell offsets of the sorted queries (n_cells + 1).
@@ -195,11 +197,12 @@ int launch_search(const GridIndex<T>& grid, const SPoint<T>* queries, const uint
 // Self-kNN over a multi-cloud batch: `pts` are all clouds' points in (cloud,
 // cell) order with cloud-local indices, `cell_start` the shared cell table;
 // output rows are global (off[c] + local index), neighbour indices local.
-// `work` points to 8 zeroed words and `ovf` to n_points words of device scratch.
+// `words`: search_batch_words(n_points) words of device scratch.
 // `chunk`: consecutive queries per work item of the search (speed only).
-int launch_search_batch(const CloudTable& ct, const uint32_t* cell_start, const SPoint<float>* pts, uint64_t n_points,
-                        uint32_t k, uint32_t* indices, float* sqr_dist, uint32_t* work, uint32_t* ovf,
-                        cudaStream_t s, uint32_t chunk = 16);
+size_t search_batch_words(uint64_t n_points);
+int launch_search_batch(const CloudTable& ct, const uint32_t* cell_start, const SPoint<float>* pts,
+                        uint64_t n_points, uint32_t k, uint32_t* indices, float* sqr_dist, uint32_t* words,
+                        cudaStream_t s, float occupancy, uint32_t chunk = 16);
 
 // Exclusive scan of G counts into out[0..G] (out[G] = total) with caller-owned
 // partials (ceil(G / 1024) words).

@@ -10,19 +10,19 @@
 // reference's. Results are the exact smallest (d^2, index) pairs: ties at equal
 // distance order by index (nanoflann keeps its tree-traversal order there).
 //
-// Two kernels:
-//  * fast_search_kernel (float, k <= 128): a warp takes chunks of 16
+// Large searches go by groups of queries first (group.cu); the queries it leaves
+// over, and smaller searches, take two kernels:
+//  * fast_search_kernel (float, k <= 128): a warp takes work items of
 //    consecutive queries in cell order. One pass over the cells within a bound
 //    tau of the query appends every point with d^2 <= tau^2 to a shared-memory
 //    buffer; selection then runs in shared memory (64-bin distance histogram,
-//    counting-sort scatter of the bins up to the k-th, insertion sort inside the
+//    counting-sort scatter of the bins up to the k-th, ranks inside the
 //    few-entry bins). For kNN, tau comes from the queries the warp solved last
 //    (one per lane): d_k(p) + |q - p| / 2 minimised over the lanes, an
 //    optimistic form of the triangle inequality d_k(q) <= d_k(p) + |q - p| that
-//    is exact whenever it holds >= k points; only the first query of a chunk
-//    needs a pilot pass; radius search uses tau = r. Queries whose buffer
-//    overflows or whose radius fell short go to a list: a second fast pass with
-//    pilot bounds, then the general kernel.
+//    is exact whenever it holds >= k points; only the first query of an item
+//    needs a pilot pass; radius search uses tau = r. A query whose buffer
+//    overflows is collected again within the bound its histogram gives.
 //  * search_kernel (float and double, any k): the general path. A pilot pass
 //    histograms a block of cells holding >= k points to bound the k-th distance,
 //    then passes over the cells within that bound refine a window of bins (first
@@ -39,6 +39,7 @@
 #include <cstdlib>
 
 #include "eig3.cuh"
+#include "group.cuh"
 #include "kernels.cuh"
 
 namespace pgeof {
@@ -158,11 +159,7 @@ __device__ __forceinline__ float axis_gap(float v, int c, float o, float h, floa
 
 // Visit every point of the cells in `bx` (rows clipped to the sphere of radius
 // Rf around q when prune). All lanes call visit(valid, d2, idx) together.
-// U > 1 loads U batches of 32 points before visiting them (U loads in flight
-// per lane: for the few, large queries of the list passes, whose warps
-// otherwise wait on one load at a time; 1M-point scene, k = 50: both list
-// passes 0.131 ms with U = 1, 0.110 ms with U = 4, 0.113 ms with U = 8).
-template <typename T, typename F, int U = 1>
+template <typename T, typename F>
 __device__ __forceinline__ void visit_box(const GridView<T>& gv, uint32_t* run_start, uint32_t* run_len,
                                           const T (&q)[3], const Box& bx, bool prune, float Rf, F&& visit) {
     const GridParams& g = gv.g;
@@ -219,37 +216,6 @@ __device__ __forceinline__ void visit_box(const GridView<T>& gv, uint32_t* run_s
         const uint32_t excl = incl - c_len;
         const uint32_t total = __shfl_sync(FULL, incl, 31);
         int r_base = 0;
-        if constexpr (U > 1) {
-            for (uint32_t base0 = 0; base0 < total; base0 += 32 * U) {
-                SPoint<T> p[U];
-                bool valid[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint32_t base = base0 + 32u * u;
-                    const uint32_t bit =
-                        (lane < nrows && excl > base && excl < base + 32) ? (1u << (excl - base)) : 0u;
-                    const uint32_t M = __reduce_or_sync(FULL, bit);
-                    const int r = r_base + __popc(M & (0xffffffffu >> (31 - lane)));
-                    const uint32_t pos = base + lane;
-                    valid[u] = pos < total;
-                    const uint32_t r_st = __shfl_sync(FULL, c_st, r);
-                    const uint32_t r_ex = __shfl_sync(FULL, excl, r);
-                    if (valid[u]) p[u] = gv.pts[r_st + (pos - r_ex)];
-                    r_base = __popc(__ballot_sync(FULL, lane < nrows && excl <= base + 32)) - 1;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    T d2 = T(0);
-                    uint32_t idx = 0;
-                    if (valid[u]) {
-                        d2 = dist2<T>(q, p[u]);
-                        idx = p[u].idx;
-                    }
-                    visit(valid[u], d2, idx);
-                }
-            }
-            continue;
-        }
         for (uint32_t base = 0; base < total; base += 32) {
             const uint32_t bit = (lane < nrows && excl > base && excl < base + 32) ? (1u << (excl - base)) : 0u;
             const uint32_t M = __reduce_or_sync(FULL, bit);
@@ -293,7 +259,7 @@ __device__ __forceinline__ void query_cell(const GridParams& g, float x, float y
 // Pilot bound on the k-th neighbour distance: grow a block of cells around
 // the query until it holds >= k points (cell counts only), then a 32-bin
 // histogram of the block's squared distances gives tau^2 >= d_k^2.
-template <typename T, int U = 1>
+template <typename T>
 __device__ __forceinline__ T pilot_tau2(const GridView<T>& gv, uint32_t* hist32, uint32_t* run_start,
                                         uint32_t* run_len, const T (&q)[3], uint32_t k) {
     const GridParams& g = gv.g;
@@ -342,7 +308,7 @@ __device__ __forceinline__ T pilot_tau2(const GridView<T>& gv, uint32_t* hist32,
             dmax = max(dmax, d2);
         }
     };
-    visit_box<T, decltype(hist)&, U>(gv, run_start, run_len, q, bx, false, 0.0f, hist);
+    visit_box<T>(gv, run_start, run_len, q, bx, false, 0.0f, hist);
     __syncwarp();
     dmax = warp_max(dmax);
     uint32_t incl = hist32[lane];
@@ -766,6 +732,7 @@ constexpr int kChunkMax = 64;
 constexpr int kChunkMin = 4;
 constexpr int kGuide = 4;
 constexpr int kSelBins = 64;     // selection histogram
+constexpr int kMaxTries = 6;     // collections of one query before the general kernel takes it
 constexpr int kMaxInBin = 24;    // larger bins (exact ties) fall back to a bitonic sort
 
 struct FastArgs {
@@ -781,7 +748,7 @@ struct FastArgs {
     uint32_t chunk;       // consecutive queries per work item (first pass): the largest
     uint32_t chunk_min;   // ... and the smallest: items shrink to remaining / guide_div
     uint32_t guide_div;
-    const uint32_t* qlist;   // LIST pass: positions in `queries` to process ...
+    const uint32_t* qlist;   // optional: positions in `queries` to process ...
     const uint32_t* qcount;  // ... and their number (device)
     uint32_t* work;
     uint32_t* ovf_list;
@@ -906,10 +873,23 @@ __device__ __forceinline__ bool select_emit(FastWarpSmem* ws, const uint64_t* ke
     return true;
 }
 
-// LIST: a second pass over the queries whose key buffer overflowed in the
-// first (a.qlist / a.qcount), each with its pilot bound -- the first pass's
-// bound came from a solved neighbour and was too loose -- and a larger buffer.
-template <bool MULTI, bool LIST, bool SEL>
+// The largest radius^2 of the bins of ws->hist (scaled by sb) up to the one that
+// holds the k-th candidate.
+__device__ __forceinline__ float tighter_tau2(const FastWarpSmem* ws, uint32_t k, float sb) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t h0 = ws->hist[2 * lane], h1 = ws->hist[2 * lane + 1];
+    uint32_t incl = h0 + h1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const uint32_t r0 = __ballot_sync(FULL, incl - h1 >= k), r1 = __ballot_sync(FULL, incl >= k);
+    const int b = min(r0 ? 2 * (__ffs(r0) - 1) : kSelBins - 1, r1 ? 2 * (__ffs(r1) - 1) + 1 : kSelBins - 1);
+    return (float)(b + 1) / sb * 1.000001f;
+}
+
+template <bool MULTI, bool SEL>
 __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -924,23 +904,20 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
         rg = sel_ring_at(ring_base + wib * sel_ring_bytes(a.sel.max_knn, a.sel.ring), a.sel.max_knn, a.sel.ring);
     }
     const uint32_t k = a.k;
-    const uint64_t m = LIST ? (uint64_t)*a.qcount : a.m;
+    const uint64_t m = a.qlist ? (uint64_t)*a.qcount : a.m;
     for (;;) {
         // Guided work items: a.chunk consecutive queries while many remain
         // (fewer chunk starts, hence fewer pilot bounds), shrinking to
         // remaining / guide_div and at least a.chunk_min towards the end, so
-        // that warps finish together. List queries are few and costly: one
-        // per item.
+        // that warps finish together.
         uint32_t start = 0, len = 1;
         if (lane == 0) {
-            if (!LIST) {
-                len = a.chunk;
-                if (a.chunk_min < a.chunk) {
-                    const uint32_t seen = __ldcg(a.work);
-                    const uint64_t rem = seen < m ? m - seen : 0;
-                    const uint64_t g = rem / a.guide_div;
-                    len = g >= a.chunk ? a.chunk : (g <= a.chunk_min ? a.chunk_min : (uint32_t)g);
-                }
+            len = a.chunk;
+            if (a.chunk_min < a.chunk) {
+                const uint32_t seen = __ldcg(a.work);
+                const uint64_t rem = seen < m ? m - seen : 0;
+                const uint64_t g = rem / a.guide_div;
+                len = g >= a.chunk ? a.chunk : (g <= a.chunk_min ? a.chunk_min : (uint32_t)g);
             }
             start = atomicAdd(a.work, len);
         }
@@ -953,7 +930,7 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
         float rx = 0.0f, ry = 0.0f, rz = 0.0f, rdk = -1.0f;
         int rci = -1;
         for (uint64_t qpos = q0; qpos < q1; ++qpos) {
-            const uint64_t qi = LIST ? (uint64_t)a.qlist[qpos] : qpos;
+            const uint64_t qi = a.qlist ? (uint64_t)a.qlist[qpos] : qpos;
             const SPoint<float> qp = a.queries[qi];
             GridView<float> gv = a.gv;
             uint64_t row_base = 0;
@@ -966,25 +943,29 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
             }
             const GridParams& g = gv.g;
             const float q[3] = {qp.x, qp.y, qp.z};
-            bool optimistic = false;  // the first try used a triangle bound
-            for (int attempt = 0; attempt < 2; ++attempt) {
+            bool optimistic = false;   // the first try used a triangle bound
+            bool guaranteed = false;   // ... which fell short: the guaranteed one now
+            float tight = -1.0f;       // a bound from the histogram of candidates that overflowed
+            uint32_t found = 0;        // radius search: points inside the radius
+            for (int attempt = 0; attempt < kMaxTries; ++attempt) {
                 float tau2;
                 bool strict;
-                if (a.mode == MODE_KNN) {
+                if (tight >= 0.0f) {
+                    tau2 = tight;
+                    strict = false;
+                } else if (a.mode == MODE_KNN) {
                     strict = false;
                     // From a solved neighbour p, d_k(q) <= d_k(p) + |q - p|. The radius
                     // used is the optimistic d_k(p) + |q - p| / 2 (best over the lanes,
                     // neighbours within 0.9 d_k(p)): when it holds >= k points the k
                     // nearest are all among them; otherwise (count < k, ~2% of the
                     // queries of the outdoor scene) the query is collected again at
-                    // once within the guaranteed d_k(p) + |q - p|. (A pilot bound for
-                    // that second try measured slower: its extra box pass costs more
-                    // than the list pass it saves.)
+                    // once within the guaranteed d_k(p) + |q - p|.
                     float bound = INFINITY;
-                    if (!LIST && rdk >= 0.0f && rci == ci) {
+                    if (rdk >= 0.0f && rci == ci) {
                         const float dx = q[0] - rx, dy = q[1] - ry, dz = q[2] - rz;
                         const float dq = sqrtf(dx * dx + dy * dy + dz * dz);
-                        if (attempt == 0) {
+                        if (!guaranteed) {
                             if (dq <= 0.9f * rdk) bound = rdk + 0.5f * dq;
                         } else {
                             bound = rdk + dq;
@@ -996,7 +977,7 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
                         const float t = bound * 1.00002f + 1e-30f + g.margin * 1e-3f;  // rounding slack
                         tau2 = t * t;
                     } else {
-                        tau2 = pilot_tau2<float, LIST ? 4 : 1>(gv, ws->hist, ws->run_start, ws->run_len, q, k);
+                        tau2 = pilot_tau2<float>(gv, ws->hist, ws->run_start, ws->run_len, q, k);
                     }
                 } else {
                     strict = true;
@@ -1021,9 +1002,9 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
                     }
                     count += __popc(mask);
                 };
-                visit_box<float, decltype(collect)&, LIST ? 4 : 1>(gv, ws->run_start, ws->run_len, q, rb, true, tf,
-                                                                   collect);
+                visit_box<float>(gv, ws->run_start, ws->run_len, q, rb, true, tf, collect);
                 __syncwarp();
+                if (tight < 0.0f) found = count;
                 const bool short_knn = a.mode == MODE_KNN && count < k;  // the optimistic radius fell short
                 const uint32_t n_sel = a.mode == MODE_KNN ? k : min(count, k);
                 const uint64_t row = a.rows_sorted ? qi : row_base + qp.idx;
@@ -1054,7 +1035,24 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
                     }
                 }
                 if (!ok) {
-                    if (attempt == 0 && optimistic && short_knn) continue;  // the guaranteed bound next
+                    if (short_knn && optimistic && !guaranteed) {
+                        guaranteed = true;
+                        continue;
+                    }
+                    // too many candidates: their histogram (of all of them, kept or
+                    // not) bounds the k-th distance far closer -- collect again.
+                    // (Instead of a list of such queries and two more launches over
+                    // it with pilot bounds and larger buffers, which took the latency
+                    // of the costliest query twice: 0.116 ms on the 1M-point scene,
+                    // 0.045 ms on 100k points; this pass pays 0.02-0.03 ms.)
+                    if (!short_knn && attempt + 1 < kMaxTries) {
+                        const float t = tighter_tau2(ws, k, sb);
+                        if (t < tau2) {
+                            tight = t;
+                            __syncwarp();
+                            continue;
+                        }
+                    }
                     if (lane == 0) {
                         const uint32_t slot = atomicAdd(a.ovf_count, 1u);
                         a.ovf_list[slot] = (uint32_t)qi;
@@ -1064,7 +1062,7 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
                 if constexpr (SEL) {
                     // park the query; its lane solves it with the others of the ring
                     if (lane == 0) {
-                        rg.found[rg.n] = count;
+                        rg.found[rg.n] = found;
                         rg.row[rg.n] = (uint32_t)row;
                     }
                     ++rg.n;
@@ -1077,9 +1075,9 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
                         oi[j] = -1;
                         if (od) od[j] = (a.fill_last && j == k - 1) ? a.r2 : 0.0f;
                     }
-                    if (a.out_found && lane == 0) a.out_found[row] = count;
+                    if (a.out_found && lane == 0) a.out_found[row] = found;
                 }
-                if (!LIST && a.mode == MODE_KNN && lane == (int)(qi & 31)) {
+                if (a.mode == MODE_KNN && lane == (int)(qpos & 31)) {
                     rdk = sqrtf(ws->kth_d2);
                     rx = q[0];
                     ry = q[1];
@@ -1094,17 +1092,16 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
     if constexpr (SEL) sel_flush_block<float>(a.sel, rg, ring_base, kFastWarps);
 }
 
-template <bool MULTI, bool LIST, bool SEL = false>
+template <bool MULTI, bool SEL = false>
 __global__ void __launch_bounds__(kFastWarps * 32) fast_search_kernel(const __grid_constant__ FastArgs a) {
-    fast_search_body<MULTI, LIST, SEL>(a);
+    fast_search_body<MULTI, SEL>(a);
 }
 
-// The single-cloud kNN pass, compiled for 10 resident blocks per SM (48
-// registers, a 24-byte spill: 1.5% faster at k = 50, 10% at k = 1 than its
-// natural 56 registers); the radius pass keeps its natural allocation (the
-// bound makes it 3-4% slower).
-__global__ void __launch_bounds__(kFastWarps * 32, 10) fast_knn_kernel(const __grid_constant__ FastArgs a) {
-    fast_search_body<false, false, false>(a);
+// The single-cloud kNN pass, compiled for 9 resident blocks per SM (56
+// registers; 100k-point scene, k = 32: 10 / 9 / 8 blocks 0.215 / 0.199 / 0.215
+// ms); the radius pass keeps its natural allocation.
+__global__ void __launch_bounds__(kFastWarps * 32, 9) fast_knn_kernel(const __grid_constant__ FastArgs a) {
+    fast_search_body<false, false>(a);
 }
 
 template <typename T>
@@ -1174,14 +1171,49 @@ int launch_general(const GridIndex<T>& grid, const SPoint<T>* queries, uint64_t 
     return launch_general_view<T>(gv, CloudTable{}, queries, m, qlist, qcount, mode, k, radius, out, s);
 }
 
-// The fast kernel over `queries` (cell order), then the general kernel over the
-// queries whose buffer overflowed. `words`: 8 + m words of scratch (work
-// counter, overflow count, overflow list). With `words2` (another 2 (8 + m)
-// words) the overflowing queries get two list passes of the fast kernel
-// (pilot bounds, 1024- then 4096-key buffers) before the general kernel.
+// Scratch words of launch_fast: counters, two lists of m entries, and the
+// grouped kernel's (16-byte aligned: the lists are rounded up).
+constexpr size_t kCtlWords = 64;
+constexpr uint64_t kOrderMin = 400000;  // queries from which the grouped kernel's leftovers are put in order
+size_t list_words(uint64_t m) { return ((size_t)m + 3) / 4 * 4; }
+size_t fast_words(uint64_t m, uint64_t block_words) {
+    return kCtlWords + 2 * list_words(m) + (group_scratch_bytes(m) + 3) / 4 + block_words;
+}
+
+// The grouped kernel (k <= kGroupMaxK), the fast kernel over
+// what it leaves over (everything without it), and the general kernel over the
+// queries whose candidates the fast kernel could not bring into its buffers.
 int launch_fast(const GridView<float>& gv, const CloudTable& ct, const SPoint<float>* queries, uint64_t m, int mode,
-                uint32_t k, float radius, const SearchOut<float>& out, uint32_t* words, uint32_t* words2,
-                cudaStream_t s, uint32_t chunk = 0) {
+                uint32_t k, float radius, const SearchOut<float>& out, uint32_t* words, cudaStream_t s,
+                float occupancy, uint64_t block_words, uint32_t chunk = 0) {
+    uint32_t* const list_a = words + kCtlWords;
+    uint32_t* const list_b = list_a + list_words(m);
+    PGEOF_CUDA_TRY(cudaMemsetAsync(words, 0, kCtlWords * sizeof(uint32_t), s));
+    // (the grouped kernel scales its bins by 1 / r^2)
+    const float r2 = radius * radius;
+    const bool grouped = occupancy > 0.0f && !out.sel && k <= kGroupMaxK && (mode == MODE_KNN || (r2 >= 1e-30f && r2 <= 1e30f));
+    if (grouped) {
+        GroupSearch gs;
+        gs.g = gv.g;
+        gs.cell_start = gv.cell_start;
+        gs.pts = gv.pts;
+        gs.ct = ct;
+        gs.queries = queries;
+        gs.m = m;
+        gs.mode = mode;
+        gs.k = k;
+        gs.radius = radius;
+        gs.occupancy = occupancy;
+        gs.counters = words + 8;
+        gs.groups = list_b + list_words(m);
+        gs.rest_count = words;
+        gs.rest = list_a;
+        if (block_words) {
+            gs.block_counts = list_b + list_words(m) + (group_scratch_bytes(m) + 3) / 4;
+            gs.rest_sorted = list_b;
+        }
+        PGEOF_TRY(launch_group_search(gs, out, s));
+    }
     const DeviceInfo* di;
     PGEOF_TRY(current_device_info(&di));
     // candidate buffer: 256 keys for kNN, 512 for radius (or 4k); selected
@@ -1200,9 +1232,9 @@ int launch_fast(const GridView<float>& gv, const CloudTable& ct, const SPoint<fl
     const int ring_smem = out.sel ? (int)(kFastWarps * sel_ring_bytes(out.sel->max_knn, out.sel->ring)) : 0;
     const int smem =
         (int)(kFastWarps * (sizeof(FastWarpSmem) + (size_t)(cap + cap_sorted) * sizeof(uint64_t))) + ring_smem;
-    auto kern = out.sel ? fast_search_kernel<false, false, true>
-                        : (ct.n ? fast_search_kernel<true, false>
-                                : (mode == MODE_KNN ? fast_knn_kernel : fast_search_kernel<false, false>));
+    auto kern = out.sel ? fast_search_kernel<false, true>
+                        : (ct.n ? fast_search_kernel<true>
+                                : (mode == MODE_KNN ? fast_knn_kernel : fast_search_kernel<false>));
     int per_sm = 0;
     PGEOF_TRY(kernel_blocks_per_sm((const void*)kern, kFastWarps * 32, smem, &per_sm));
     // Queries per work item: a fixed count when the caller gives one (batch
@@ -1226,7 +1258,6 @@ int launch_fast(const GridView<float>& gv, const CloudTable& ct, const SPoint<fl
     const uint32_t chunk_min = chunk ? chunk : std::min(guided_min, guided_max);
     const uint64_t items = ceil_div_u(m, chunk_min);
     const uint64_t blocks = std::min<uint64_t>(ceil_div_u(items, kFastWarps), (uint64_t)di->sm_count * per_sm);
-    PGEOF_CUDA_TRY(cudaMemsetAsync(words, 0, 8 * sizeof(uint32_t), s));
     FastArgs a{};
     a.gv = gv;
     a.ct = ct;
@@ -1245,9 +1276,13 @@ int launch_fast(const GridView<float>& gv, const CloudTable& ct, const SPoint<fl
         return (uint64_t)std::min<unsigned long>(std::max<unsigned long>(v, 1ul), 64ul);
     }();
     a.guide_div = (uint32_t)std::max<uint64_t>(1, guide * blocks * kFastWarps);
-    a.work = words;
-    a.ovf_count = words + 1;
-    a.ovf_list = words + 8;
+    if (grouped) {
+        a.qlist = block_words ? list_b : list_a;
+        a.qcount = words;
+    }
+    a.work = words + 2;
+    a.ovf_count = words + 3;
+    a.ovf_list = a.qlist == list_b ? list_a : list_b;  // (each pass reads one list and writes the other)
     a.out_idx = out.indices;
     a.out_d2 = out.sqr_dist;
     a.out_found = out.found;
@@ -1262,45 +1297,6 @@ int launch_fast(const GridView<float>& gv, const CloudTable& ct, const SPoint<fl
     }
     count_launch();
     PGEOF_TRY(check_launch("fast_search_kernel"));
-    if (words2 && !ct.n) {
-        // List passes over the overflowing queries (one query per work item,
-        // a pilot bound, a larger buffer), sized on the device: 1024 keys, then
-        // 4096 keys for the few that still overflow, and the general kernel
-        // (refinement passes) for whatever is left -- usually nothing. The
-        // small first list buffer keeps that pass's occupancy for its
-        // thousands of queries; the second pass spares the general kernel's
-        // refinement passes, whose latency made its launch long.
-        const uint32_t* in_list = a.ovf_list;
-        const uint32_t* in_count = a.ovf_count;
-        for (int pass = 0; pass < 2; ++pass) {
-            uint32_t* w = words2 + (size_t)pass * (m + 8);
-            uint32_t cap2 = 1;
-            while (cap2 < std::max<uint64_t>(pass == 0 ? 1024 : 4096, 4ull * k)) cap2 <<= 1;
-            const int smem2 =
-                (int)(kFastWarps * (sizeof(FastWarpSmem) + (size_t)(cap2 + cap_sorted) * sizeof(uint64_t))) +
-                ring_smem;
-            auto kern2 = out.sel ? fast_search_kernel<false, true, true> : fast_search_kernel<false, true>;
-            int per_sm2 = 0;
-            PGEOF_TRY(kernel_blocks_per_sm((const void*)kern2, kFastWarps * 32, smem2, &per_sm2));
-            PGEOF_CUDA_TRY(cudaMemsetAsync(w, 0, 8 * sizeof(uint32_t), s));
-            FastArgs a2 = a;
-            a2.cap = cap2;
-            a2.qlist = in_list;
-            a2.qcount = in_count;
-            a2.work = w;
-            a2.ovf_count = w + 1;
-            a2.ovf_list = w + 8;
-            {
-                KernelTimer kt("overflow_list_kernel", s);
-                kern2<<<(unsigned)((uint64_t)di->sm_count * per_sm2), kFastWarps * 32, smem2, s>>>(a2);
-            }
-            count_launch();
-            PGEOF_TRY(check_launch("fast_search_kernel(list)"));
-            in_list = a2.ovf_list;
-            in_count = a2.ovf_count;
-        }
-        return launch_general_view<float>(gv, ct, queries, m, in_list, in_count, mode, k, radius, out, s);
-    }
     // queries whose key buffer overflowed: the general kernel, sized on the device
     return launch_general_view<float>(gv, ct, queries, m, a.ovf_list, a.ovf_count, mode, k, radius, out, s);
 }
@@ -1318,19 +1314,23 @@ int launch_search(const GridIndex<T>& grid, const SPoint<T>* queries, const uint
         if (k > 128 || m >= 0xfff00000ull)  // 32-bit work counters with headroom for the last items
             return launch_general<T>(grid, queries, m, nullptr, nullptr, mode, k, radius, out, s);
         Scratch ctl;
-        PGEOF_TRY(ctl.alloc(3 * (m + 8) * sizeof(uint32_t), s));
+        const float occupancy = use_groups(grid.n, m, k) ? grid.grouped : 0.0f;
+        const uint64_t block_words = occupancy > 0.0f && m >= kOrderMin ? group_block_words(grid.g) : 0;
+        PGEOF_TRY(ctl.alloc(fast_words(m, block_words) * sizeof(uint32_t), s));
         GridView<float> gv;
         gv.g = grid.g;
         gv.cell_start = grid.cell_start;
         gv.pts = grid.pts;
-        return launch_fast(gv, CloudTable{}, queries, m, mode, k, radius, out, ctl.as<uint32_t>(),
-                           ctl.as<uint32_t>() + m + 8, s);
+        return launch_fast(gv, CloudTable{}, queries, m, mode, k, radius, out, ctl.as<uint32_t>(), s, occupancy,
+                           block_words);
     }
 }
 
+size_t search_batch_words(uint64_t n_points) { return fast_words(n_points, 0); }
+
 int launch_search_batch(const CloudTable& ct, const uint32_t* cell_start, const SPoint<float>* pts, uint64_t n_points,
-                        uint32_t k, uint32_t* indices, float* sqr_dist, uint32_t* work, uint32_t* ovf,
-                        cudaStream_t s, uint32_t chunk) {
+                        uint32_t k, uint32_t* indices, float* sqr_dist, uint32_t* words, cudaStream_t s,
+                        float occupancy, uint32_t chunk) {
     if (n_points == 0 || k == 0) return PGEOF_OK;
     GridView<float> gv{};
     gv.cell_start = cell_start;
@@ -1340,8 +1340,7 @@ int launch_search_batch(const CloudTable& ct, const uint32_t* cell_start, const 
     out.sqr_dist = sqr_dist;
     if (k > 128)
         return launch_general_view<float>(gv, ct, pts, n_points, nullptr, nullptr, MODE_KNN, k, 0.0f, out, s);
-    (void)ovf;
-    return launch_fast(gv, ct, pts, n_points, MODE_KNN, k, 0.0f, out, work, nullptr, s, chunk);
+    return launch_fast(gv, ct, pts, n_points, MODE_KNN, k, 0.0f, out, words, s, occupancy, 0, chunk);
 }
 
 template int launch_search<float>(const GridIndex<float>&, const SPoint<float>*, const uint32_t*, uint64_t, int,
