@@ -440,8 +440,9 @@ __global__ void pad_xyz_kernel(const float* __restrict__ xyz, uint64_t n, float4
 }
 
 // ------------------------------------------------------------------ optimal
-constexpr int kOptThreads = 128;
-constexpr int kOptSlots = 64;  // eigentropy values kept per point for the near-tie pass
+constexpr int kOptThreads = 64;
+constexpr int kOptCands = 8;       // near-tied sizes kept per point
+constexpr uint32_t kOptSizes = 64;  // points with more candidate sizes have all of them evaluated exactly
 
 struct OptArgs {
     const float4* xyz4;
@@ -455,71 +456,99 @@ struct OptArgs {
     float* out;  // (n, 12)
     uint32_t* err;
     unsigned long long* stats;  // [0] exact tie re-evaluations, [1] double re-solves
+    // rows left to optimal_exact_kernel: their number, then the rows; a queued
+    // output row carries the number of near-tied sizes and the sizes themselves
+    uint32_t* queue;
 };
 
-// Kahan-compensated running sum.
-struct KSum {
-    float s = 0.0f, c = 0.0f;
-    __device__ __forceinline__ void add(float x) {
-        const float y = FSUB(x, c);
-        const float t = FADD(s, y);
-        c = FSUB(FSUB(t, s), y);
+// Packed pairs of floats: one instruction for two values, each rounded as its
+// scalar form.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    return ((F2)__float_as_uint(hi) << 32) | __float_as_uint(lo);
+}
+__device__ __forceinline__ float f2_lo(F2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float f2_hi(F2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {  // a - b
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+    return r;
+}
+
+// Two Kahan-compensated running sums.
+struct KSum2 {
+    F2 s = 0, c = 0;
+    __device__ __forceinline__ void add(F2 x) {
+        const F2 y = f2_sub(x, c);
+        const F2 t = f2_add(s, y);
+        c = f2_sub(f2_sub(t, s), y);
         s = t;
     }
 };
 
-// Eigenvalues of a symmetric 3x3 by the trigonometric closed form (O. K.
-// Smith, "Eigenvalues of a symmetric 3x3 matrix", CACM 4(4), 1961), used only
-// to rank candidate neighbourhood sizes. The scan ranks candidate sizes and every size within
-// kTieBand (3e-5) of its minimum is re-evaluated exactly, so the scan's values
-// need only stay within half the band of the exact ones. The hardware cosine
-// and logarithm (__cosf: absolute error < 2^-21 on [-pi, pi]; __logf) add about
-// 1e-6 to the eigentropy -- well inside it.
-__device__ __forceinline__ void eigvals_closed_form_scan(const Cov<float>& c, float (&w)[3]) {
+// Eigentropy (include/pca.hpp:140-150) of a covariance for ranking candidate
+// sizes: the trigonometric closed form of the eigenvalues (O. K. Smith,
+// "Eigenvalues of a symmetric 3x3 matrix", CACM 4(4), 1961). Every size within
+// kTieBand (3e-5) of the minimum is re-evaluated exactly, so these values need
+// only stay within half the band of the exact ones. The arc cosine is
+// Abramowitz & Stegun 4.4.46 (error <= 2e-8) and the other functions are the
+// hardware's (__cosf: absolute error < 2^-21 on [-pi, pi]; __logf): about 1e-6
+// in the eigentropy.
+__device__ __forceinline__ float eigentropy_scan(const Cov<float>& c) {
     const float q = (c.xx + c.yy + c.zz) * (1.0f / 3.0f);
     const float b00 = c.xx - q, b11 = c.yy - q, b22 = c.zz - q;
     const float off = c.xy * c.xy + c.xz * c.xz + c.yz * c.yz;
-    const float p2 = (b00 * b00 + b11 * b11 + b22 * b22 + 2.0f * off) * (1.0f / 6.0f);
-    if (!(p2 > 0.0f)) {
-        w[0] = w[1] = w[2] = q;
-        return;
-    }
-    const float p = sqrtf(p2);
+    const float p2 = fmaxf((b00 * b00 + b11 * b11 + b22 * b22 + 2.0f * off) * (1.0f / 6.0f), 1e-36f);
+    float inv_p = rsqrtf(p2);
+    inv_p *= fmaf(-0.5f * p2 * inv_p, inv_p, 1.5f);  // (its cube goes into r, which near 1 loses half its digits below)
+    const float p = p2 * inv_p;
     const float det = b00 * (b11 * b22 - c.yz * c.yz) - c.xy * (c.xy * b22 - c.yz * c.xz) +
                       c.xz * (c.xy * c.yz - b11 * c.xz);
-    float r = __fdividef(det, 2.0f * p2 * p);
-    r = fminf(1.0f, fmaxf(-1.0f, r));
-    const float phi = acosf(r) * (1.0f / 3.0f);
+    const float r = fminf(1.0f, fmaxf(-1.0f, det * (0.5f * inv_p) * inv_p * inv_p));
+    const float x = fabsf(r);
+    float a = -0.0012624911f;
+    a = fmaf(a, x, 0.0066700901f);
+    a = fmaf(a, x, -0.0170881256f);
+    a = fmaf(a, x, 0.0308918810f);
+    a = fmaf(a, x, -0.0501743046f);
+    a = fmaf(a, x, 0.0889789874f);
+    a = fmaf(a, x, -0.2145988016f);
+    a = fmaf(a, x, 1.5707963050f);
+    const float y = 1.0f - x;
+    a *= y > 0.0f ? y * rsqrtf(y) : 0.0f;
+    const float phi = (r < 0.0f ? 3.14159265f - a : a) * (1.0f / 3.0f);
     const float e2 = q + 2.0f * p * __cosf(phi);
     const float e0 = q + 2.0f * p * __cosf(phi + 2.0943951023931953f);
-    w[0] = e0;
-    w[2] = e2;
-    w[1] = 3.0f * q - e0 - e2;
-}
-
-// include/pca.hpp:140-150 with the hardware logarithm (scan ranking only).
-__device__ __forceinline__ float eigentropy_scan(const float (&val)[3]) {
+    const float e1 = 3.0f * q - e0 - e2;
+    const float v0 = fmaxf(e0, 0.0f), v1 = fmaxf(e1, 0.0f), v2 = fmaxf(e2, 0.0f);
     const float eps = 1e-3f;
-    const float inv = __fdividef(1.0f, val[0] + val[1] + val[2] + eps);
-    const float e0 = val[0] * inv, e1 = val[1] * inv, e2 = val[2] * inv;
-    return -(e0 * __logf(e0 + eps) + e1 * __logf(e1 + eps) + e2 * __logf(e2 + eps));
+    const float inv = __fdividef(1.0f, v0 + v1 + v2 + eps);
+    const float f0 = v0 * inv, f1 = v1 * inv, f2 = v2 * inv;
+    return -(f0 * __logf(f0 + eps) + f1 * __logf(f1 + eps) + f2 * __logf(f2 + eps));
 }
 
 // Covariance of the first k neighbours exactly as include/pca.hpp:75-76.
 __device__ __forceinline__ Cov<float> literal_cov(const OptArgs& a, uint32_t b, uint32_t k, uint32_t& flags) {
-    // scalar index loads here: the 4-wide form costs this kernel ~20 registers
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    for (uint32_t j = 0; j < k; ++j) {
-        const float4 p = gather_nb(a.xyz4, a.n_xyz, __ldg(a.nn + b + j), flags);
+    gather_row(a.nn, b, k, a.xyz4, a.n_xyz, flags, [&](uint32_t, const float4& p) {
         sx = FADD(sx, p.x);
         sy = FADD(sy, p.y);
         sz = FADD(sz, p.z);
-    }
+    });
     const float kk = (float)k;
     const float mx = FDIV(sx, kk), my = FDIV(sy, kk), mz = FDIV(sz, kk);
     float xx = 0.0f, xy = 0.0f, xz = 0.0f, yy = 0.0f, yz = 0.0f, zz = 0.0f;
-    for (uint32_t j = 0; j < k; ++j) {
-        const float4 p = gather_nb(a.xyz4, a.n_xyz, __ldg(a.nn + b + j), flags);
+    gather_row(a.nn, b, k, a.xyz4, a.n_xyz, flags, [&](uint32_t, const float4& p) {
         const float dx = FSUB(p.x, mx), dy = FSUB(p.y, my), dz = FSUB(p.z, mz);
         xx = FADD(xx, FMUL(dx, dx));
         xy = FADD(xy, FMUL(dx, dy));
@@ -527,7 +556,7 @@ __device__ __forceinline__ Cov<float> literal_cov(const OptArgs& a, uint32_t b, 
         yy = FADD(yy, FMUL(dy, dy));
         yz = FADD(yz, FMUL(dy, dz));
         zz = FADD(zz, FMUL(dz, dz));
-    }
+    });
     Cov<float> c;
     c.xx = FDIV(xx, kk);
     c.xy = FDIV(xy, kk);
@@ -538,9 +567,112 @@ __device__ __forceinline__ Cov<float> literal_cov(const OptArgs& a, uint32_t b, 
     return c;
 }
 
-__device__ __forceinline__ bool evaluated(uint32_t k, uint32_t k0, uint32_t k_nn, uint32_t step) {
-    return k == k0 || k % step == 0 || k == k_nn;
+// The reference's float eigentropy of the first k neighbours: its own
+// covariance, an exact eigen solve.
+__device__ __noinline__ float exact_eigentropy(const OptArgs& a, uint32_t b, uint32_t k, uint32_t& flags) {
+    Pca<float> p;
+    pca_solve_f64<float>(literal_cov(a, b, k, flags), a.order, &p);
+    return eigentropy_of<float>(p.val);
 }
+
+// Calls f(k, dx, dy, dz) for k = 1 .. k_nn: neighbour k's offset from the first
+// one. Neighbours go by aligned groups of four indices (one 16-byte read where
+// the group lies inside nn), and the next group's points are on their way while
+// four are handled. f appears once in the code: four copies of a scan's step
+// ran out of the instruction cache (3.4 of 9 stall cycles per instruction).
+template <typename F>
+__device__ __forceinline__ void offset_row(const OptArgs& a, uint32_t b, uint32_t k_nn, uint32_t& flags, F&& f) {
+    const uint32_t* row = a.nn + b;
+    const uint32_t id0 = __ldg(row);
+    const float4 p0 = gather_nb(a.xyz4, a.n_xyz, id0, flags);
+    const int skip = (int)((reinterpret_cast<uintptr_t>(row) >> 2) & 3u);  // places of the first group before the row
+    const int end = (int)k_nn;
+    const auto indices = [&](int j) {  // of places j .. j + 3 of the row (j + skip a multiple of 4)
+        const uint32_t* g = row + j;
+        if (g >= a.nn && g + 4 <= a.nn + a.nnz) {
+            uint4 v = __ldg(reinterpret_cast<const uint4*>(g));
+            if (j < 0 || j + 4 > end) {
+                if (j < 0) v.x = id0;
+                if ((uint32_t)(j + 1) >= k_nn) v.y = id0;
+                if ((uint32_t)(j + 2) >= k_nn) v.z = id0;
+                if ((uint32_t)(j + 3) >= k_nn) v.w = id0;
+            }
+            return v;
+        }
+        uint4 v;
+        v.x = (uint32_t)j < k_nn ? __ldg(g) : id0;
+        v.y = (uint32_t)(j + 1) < k_nn ? __ldg(g + 1) : id0;
+        v.z = (uint32_t)(j + 2) < k_nn ? __ldg(g + 2) : id0;
+        v.w = (uint32_t)(j + 3) < k_nn ? __ldg(g + 3) : id0;
+        return v;
+    };
+    uint4 ids = indices(-skip);
+    float4 q0 = gather_nb(a.xyz4, a.n_xyz, ids.x, flags), q1 = gather_nb(a.xyz4, a.n_xyz, ids.y, flags);
+    float4 q2 = gather_nb(a.xyz4, a.n_xyz, ids.z, flags), q3 = gather_nb(a.xyz4, a.n_xyz, ids.w, flags);
+    if (4 - skip < end) ids = indices(4 - skip);
+    for (int j = -skip; j < end;) {
+        float4 c0 = q0, c1 = q1, c2 = q2, c3 = q3;
+        if (j + 4 < end) {
+            q0 = gather_nb(a.xyz4, a.n_xyz, ids.x, flags);
+            q1 = gather_nb(a.xyz4, a.n_xyz, ids.y, flags);
+            q2 = gather_nb(a.xyz4, a.n_xyz, ids.z, flags);
+            q3 = gather_nb(a.xyz4, a.n_xyz, ids.w, flags);
+            if (j + 8 < end) ids = indices(j + 8);
+        }
+#pragma unroll 1
+        for (int t = 0; t < 4; ++t, ++j) {
+            if ((uint32_t)j < k_nn) f((uint32_t)j + 1, c0.x - p0.x, c0.y - p0.y, c0.z - p0.z);
+            c0 = c1;
+            c1 = c2;
+            c2 = c3;
+        }
+    }
+}
+
+// The compensated prefix moments of offset_row's points.
+struct Moments {
+    KSum2 s_xy, s_z, s_xx_xy, s_xz_yz, s_yy_zz;
+    __device__ __forceinline__ void add(float dx, float dy, float dz) {
+        const F2 d01 = f2(dx, dy), d12 = f2(dy, dz);
+        s_xy.add(d01);
+        s_z.add(f2(dz, 0.0f));
+        s_xx_xy.add(f2_mul(f2(dx, dx), d01));
+        s_xz_yz.add(f2_mul(d01, f2(dz, dz)));
+        s_yy_zz.add(f2_mul(d12, d12));
+    }
+    __device__ __forceinline__ Cov<float> cov(uint32_t k) const {
+        const float inv = __fdividef(1.0f, (float)k);
+        const float mx = f2_lo(s_xy.s) * inv, my = f2_hi(s_xy.s) * inv, mz = f2_lo(s_z.s) * inv;
+        Cov<float> c;
+        c.xx = f2_lo(s_xx_xy.s) * inv - mx * mx;
+        c.xy = f2_hi(s_xx_xy.s) * inv - mx * my;
+        c.xz = f2_lo(s_xz_yz.s) * inv - mx * mz;
+        c.yy = f2_lo(s_yy_zz.s) * inv - my * my;
+        c.yz = f2_hi(s_xz_yz.s) * inv - my * mz;
+        c.zz = f2_hi(s_yy_zz.s) * inv - mz * mz;
+        return c;
+    }
+};
+
+// The sizes of a row: k0, the multiples of k_step above it, and k_nn.
+struct Sizes {
+    uint32_t k0, step, k_nn, due;
+    __device__ __forceinline__ Sizes(const OptArgs& a, uint32_t k_nn_)
+        : k0(min(max(a.k_min, a.k_min_search), k_nn_)), step(a.k_step), k_nn(k_nn_), due(k0) {}
+    __device__ __forceinline__ uint32_t count() const {
+        const uint32_t multiples = k_nn / step - k0 / step;  // in (k0, k_nn]
+        return 1 + multiples + (k_nn > k0 && k_nn % step != 0);
+    }
+    __device__ __forceinline__ bool take(uint32_t k) {  // (called for k = 1, 2, ...)
+        if (k == due) {
+            due = step == 1 ? k + 1 : (k / step + 1) * step;
+            return true;
+        }
+        return k == k_nn;
+    }
+};
+
+constexpr float kTieBand = 3e-5f;
 
 // include/pgeof.hpp:264-299. Candidate sizes are ranked by eigentropy from
 // compensated prefix moments (O(k) gathers instead of the reference's O(k^2));
@@ -548,17 +680,26 @@ __device__ __forceinline__ bool evaluated(uint32_t k, uint32_t k0, uint32_t k_nn
 // then re-evaluated from the reference's own covariance and an exact eigen
 // solve, and the smallest exact eigentropy wins (first k on equality -- the
 // reference's strict '<' scan). Features come from the winning size's
-// reference covariance.
-__global__ void __launch_bounds__(kOptThreads) optimal_kernel(const __grid_constant__ OptArgs a) {
-    constexpr float kTieBand = 3e-5f;
-    __shared__ float ent[kOptSlots * kOptThreads];
+// reference covariance. Rows that need an exact solve (near-tied sizes, 0.4% of
+// a scene's; small eigen-gaps) are queued for optimal_exact_kernel.
+//
+// What bounds it: instruction issue (68% of slots), after the gathers' latency
+// and L1 look-ups in the scan (one random 16-byte read per neighbour). So four
+// points are in flight per thread while four are handled, indices come four at
+// a time, moments are summed in packed pairs, and only near-tied sizes are kept
+// (one eigentropy per size took 32 KB of shared memory a block and half the
+// resident warps). 4M rows of up to 64 neighbours: 5.98 -> 3.16 ms, and 0.22 ms
+// for the queue. Blocks of 64 x 12 / 128 x 6 / 128 x 5 / 32 x 20 per SM: 3.16 /
+// 3.20 / 3.29 / 3.22 ms.
+__global__ void __launch_bounds__(kOptThreads, 12) optimal_kernel(const __grid_constant__ OptArgs a) {
+    __shared__ float cand_e[kOptCands * kOptThreads];
+    __shared__ uint32_t cand_k[kOptCands * kOptThreads];
     __shared__ float stage[12 * kOptThreads];
     const int tid = threadIdx.x;
     const uint32_t i = blockIdx.x * kOptThreads + tid;
 #pragma unroll
     for (int f = 0; f < 12; ++f) stage[f * kOptThreads + tid] = 0.0f;
     uint32_t flags = 0;
-    unsigned n_exact = 0, n_resolved = 0;
     if (i < a.n_points) {
         const uint32_t b = __ldg(a.ptr + i), e = __ldg(a.ptr + i + 1);
         uint32_t k_nn = 0;
@@ -570,111 +711,63 @@ __global__ void __launch_bounds__(kOptThreads) optimal_kernel(const __grid_const
             k_nn = e - b;
         }
         if (ok && k_nn >= a.k_min && k_nn >= a.k_min_search && k_nn > 0) {
-            uint32_t k0 = max(a.k_min, a.k_min_search);
-            k0 = min(k0, k_nn);
-            // fast scan over prefix moments, shifted by the first neighbour
-            uint32_t id0 = __ldg(a.nn + b);
-            if (id0 >= a.n_xyz) {
-                flags |= ERR_NN_RANGE;
-                id0 = 0;
+            Sizes sizes(a, k_nn);
+            int cands = kOptCands + 1;
+            if (sizes.count() <= kOptSizes) {
+                cands = 0;
+                float best = INFINITY;
+                Moments m;
+                offset_row(a, b, k_nn, flags, [&](uint32_t k, float dx, float dy, float dz) {
+                    m.add(dx, dy, dz);
+                    if (!sizes.take(k)) return;
+                    const float ent = eigentropy_scan(m.cov(k));
+                    if (!(ent <= best + kTieBand)) return;
+                    if (ent < best) {
+                        const bool far = !(best <= ent + kTieBand);  // no earlier size is near-tied any more
+                        best = ent;
+                        int kept = 0;
+                        for (int t = 0; t < min(cands, kOptCands); ++t) {
+                            const float et = cand_e[t * kOptThreads + tid];
+                            if (et <= best + kTieBand) {
+                                cand_e[kept * kOptThreads + tid] = et;
+                                cand_k[kept * kOptThreads + tid] = cand_k[t * kOptThreads + tid];
+                                ++kept;
+                            }
+                        }
+                        cands = cands > kOptCands && !far ? kOptCands + 1 : kept;
+                    }
+                    if (cands < kOptCands) {
+                        cand_e[cands * kOptThreads + tid] = ent;
+                        cand_k[cands * kOptThreads + tid] = k;
+                    }
+                    cands = min(cands + 1, kOptCands + 1);
+                });
             }
-            const float4 p0 = __ldg(a.xyz4 + id0);
-            KSum s1x, s1y, s1z, sxx, sxy, sxz, syy, syz, szz;
-            float best = 0.0f;
-            int slot = 0;
-            bool stored_all = true;
-            for (uint32_t k = 1; k <= k_nn; ++k) {
-                const float4 p = gather_nb(a.xyz4, a.n_xyz, __ldg(a.nn + b + k - 1), flags);
-                const float dx = p.x - p0.x, dy = p.y - p0.y, dz = p.z - p0.z;
-                s1x.add(dx);
-                s1y.add(dy);
-                s1z.add(dz);
-                sxx.add(dx * dx);
-                sxy.add(dx * dy);
-                sxz.add(dx * dz);
-                syy.add(dy * dy);
-                syz.add(dy * dz);
-                szz.add(dz * dz);
-                if (k < k0 || !evaluated(k, k0, k_nn, a.k_step)) continue;
-                const float inv = 1.0f / (float)k;
-                const float mx = s1x.s * inv, my = s1y.s * inv, mz = s1z.s * inv;
-                Cov<float> c;
-                c.xx = sxx.s * inv - mx * mx;
-                c.xy = sxy.s * inv - mx * my;
-                c.xz = sxz.s * inv - mx * mz;
-                c.yy = syy.s * inv - my * my;
-                c.yz = syz.s * inv - my * mz;
-                c.zz = szz.s * inv - mz * mz;
-                float w[3];
-                eigvals_closed_form_scan(c, w);
-                float val[3];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) val[q] = fmaxf(w[a.order ? 2 - q : q], 0.0f);
-                const float ent_k = eigentropy_scan(val);
-                if (k == k0 || ent_k < best) best = ent_k;
-                if (slot < kOptSlots) {
-                    ent[slot * kOptThreads + tid] = ent_k;
+            bool queued = cands > 1;
+            if (!queued) {
+                const uint32_t k_opt = cands == 1 ? cand_k[tid] : sizes.k0;
+                Pca<float> p;
+                queued = !pca_solve_f32_fast(literal_cov(a, b, k_opt, flags), a.order, p);
+                if (queued) {
+                    cands = 1;
+                    cand_k[tid] = k_opt;
                 } else {
-                    stored_all = false;
-                }
-                ++slot;
-            }
-            // candidates within the tie band of the fast minimum
-            int n_cand = 0;
-            for (int sidx = 0; sidx < min(slot, kOptSlots); ++sidx)
-                if (ent[sidx * kOptThreads + tid] <= best + kTieBand) ++n_cand;
-            uint32_t k_opt = k0;
-            if (stored_all && n_cand == 1) {
-                // unique winner: find its k
-                int sidx = 0;
-                for (uint32_t k = k0; k <= k_nn; ++k) {
-                    if (!evaluated(k, k0, k_nn, a.k_step)) continue;
-                    if (ent[sidx * kOptThreads + tid] <= best + kTieBand) {
-                        k_opt = k;
-                        break;
-                    }
-                    ++sidx;
-                }
-            } else {
-                // near-ties (or too many sizes to store): exact re-evaluation
-                float best_exact = 0.0f;
-                bool have = false;
-                int sidx = 0;
-                for (uint32_t k = k0; k <= k_nn; ++k) {
-                    if (!evaluated(k, k0, k_nn, a.k_step)) continue;
-                    bool cand = true;
-                    if (stored_all) cand = ent[sidx * kOptThreads + tid] <= best + kTieBand;
-                    ++sidx;
-                    if (!cand) continue;
-                    ++n_exact;
-                    const Cov<float> c = literal_cov(a, b, k, flags);
-                    Pca<float> pk;
-                    pca_solve_f64<float>(c, a.order, &pk);
-                    const float ek = eigentropy_of<float>(pk.val);
-                    if (!have || ek < best_exact) {
-                        best_exact = ek;
-                        k_opt = k;
-                        have = true;
-                    }
-                }
-            }
-            const Cov<float> c = literal_cov(a, b, k_opt, flags);
-            Pca<float> p;
-            bool res;
-            pca_solve_f32(c, a.order, p, res);
-            n_resolved += res;
-            float f[11];
-            features11(p, f);
+                    float f[11];
+                    features11(p, f);
 #pragma unroll
-            for (int q = 0; q < 11; ++q) stage[q * kOptThreads + tid] = f[q];
-            stage[11 * kOptThreads + tid] = (float)k_opt;
+                    for (int q = 0; q < 11; ++q) stage[q * kOptThreads + tid] = f[q];
+                    stage[11 * kOptThreads + tid] = (float)k_opt;
+                }
+            }
+            if (queued) {
+                a.queue[1 + atomicAdd(a.queue, 1u)] = i;
+                stage[tid] = __uint_as_float((uint32_t)cands);
+                for (int t = 0; t < min(cands, kOptCands); ++t)
+                    stage[(1 + t) * kOptThreads + tid] = __uint_as_float(cand_k[t * kOptThreads + tid]);
+            }
         }
     }
     if (flags) atomicOr(a.err, flags);
-    if (a.stats) {
-        if (n_exact) atomicAdd(a.stats, (unsigned long long)n_exact);
-        if (n_resolved) atomicAdd(a.stats + 1, (unsigned long long)n_resolved);
-    }
     __syncthreads();
     const uint32_t row0 = blockIdx.x * kOptThreads;
     const uint32_t rows = min((uint32_t)kOptThreads, a.n_points - row0);
@@ -682,6 +775,87 @@ __global__ void __launch_bounds__(kOptThreads) optimal_kernel(const __grid_const
     for (int t = tid; t < (int)rows * 12; t += kOptThreads) {
         const int r = t / 12, c = t - r * 12;
         dst[t] = stage[c * kOptThreads + r];
+    }
+}
+
+// The rows optimal_kernel queued, two lanes per row: exact eigentropies of the
+// near-tied sizes (of every size where they found no room), every other size
+// each, and an exact solve of the winner where its eigen-gap is small. A float64
+// solve is a ~40 us chain of dependent operations; the queue's solves run side
+// by side instead of holding up one warp in eight (4M rows: 0.77 ms inside
+// optimal_kernel, 0.23 ms with one lane per row).
+__global__ void __launch_bounds__(64) optimal_exact_kernel(const __grid_constant__ OptArgs a) {
+    const uint32_t n = a.queue[0], half = threadIdx.x & 1u;
+    const uint32_t step = gridDim.x * (blockDim.x / 2);
+    for (uint32_t q0 = blockIdx.x * (blockDim.x / 2); q0 < n; q0 += step) {
+        const uint32_t q = q0 + threadIdx.x / 2;
+        const bool valid = q < n;
+        const uint32_t i = a.queue[1 + (valid ? q : q0)];
+        float* out = a.out + (uint64_t)i * 12;
+        const uint32_t b = __ldg(a.ptr + i), k_nn = __ldg(a.ptr + i + 1) - b;
+        uint32_t flags = 0, n_exact = 0;
+        const int cands = valid ? (int)__float_as_uint(out[0]) : 0;
+        Sizes sizes(a, k_nn);
+        uint32_t k_opt = 0xffffffffu;
+        float best = INFINITY;
+        if (cands == 1) {
+            k_opt = __float_as_uint(out[1]);
+        } else if (cands > 1) {
+            uint32_t turn = 0;
+            const auto eval = [&](uint32_t k) {
+                if ((turn++ & 1u) != half) return;
+                const float ent = exact_eigentropy(a, b, k, flags);
+                ++n_exact;
+                if (k_opt == 0xffffffffu || ent < best) {
+                    best = ent;
+                    k_opt = k;
+                }
+            };
+            if (cands <= kOptCands) {
+                for (int t = 0; t < cands; ++t) eval(__float_as_uint(out[1 + t]));
+            } else if (sizes.count() > kOptSizes) {
+                for (uint32_t k = 1; k <= k_nn; ++k)
+                    if (sizes.take(k)) eval(k);
+            } else {
+                // the scan again for its minimum, then once more for the sizes near it
+                float low = INFINITY;
+                for (int pass = 0; pass < 2; ++pass) {
+                    Moments m;
+                    Sizes each(a, k_nn);
+                    offset_row(a, b, k_nn, flags, [&](uint32_t k, float dx, float dy, float dz) {
+                        m.add(dx, dy, dz);
+                        if (!each.take(k)) return;
+                        const float ent = eigentropy_scan(m.cov(k));
+                        if (pass == 0) low = fminf(low, ent);
+                        else if (ent <= low + kTieBand) eval(k);
+                    });
+                }
+            }
+        }
+        __syncwarp();
+        // the smaller eigentropy of the two lanes', the smaller size on equality
+        // (a NaN never replaces what came before it)
+        const float other = __shfl_xor_sync(0xffffffffu, best, 1);
+        const uint32_t other_k = __shfl_xor_sync(0xffffffffu, k_opt, 1);
+        const uint32_t first_k = min(k_opt, other_k), last_k = max(k_opt, other_k);
+        const float first = k_opt <= other_k ? best : other, last = k_opt <= other_k ? other : best;
+        k_opt = last_k != 0xffffffffu && last < first ? last_k : first_k;
+        if (flags) atomicOr(a.err, flags);
+        if (a.stats && n_exact) atomicAdd(a.stats, (unsigned long long)n_exact);
+        if (valid && half == 0) {
+            flags = 0;
+            if (k_opt == 0xffffffffu) k_opt = sizes.k0;
+            Pca<float> p;
+            bool res;
+            pca_solve_f32(literal_cov(a, b, k_opt, flags), a.order, p, res);
+            float f[11];
+            features11(p, f);
+#pragma unroll
+            for (int t = 0; t < 11; ++t) out[t] = f[t];
+            out[11] = (float)k_opt;
+            if (flags) atomicOr(a.err, flags);
+            if (a.stats && res) atomicAdd(a.stats + 1, 1ull);
+        }
     }
 }
 
@@ -846,10 +1020,22 @@ int launch_optimal(const float4* xyz4, uint64_t n_xyz, const uint32_t* nn, uint6
     a.out = out;
     a.err = device_error_word();
     a.stats = stats;
-    KernelTimer kt("optimal_kernel", s);
-    optimal_kernel<<<ceil_div_u(n_points, kOptThreads), kOptThreads, 0, s>>>(a);
+    Scratch queue;
+    PGEOF_TRY(queue.alloc((n_points + 1) * sizeof(uint32_t), s));
+    a.queue = queue.as<uint32_t>();
+    PGEOF_CUDA_TRY(cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), s));
+    const DeviceInfo* di;
+    PGEOF_TRY(current_device_info(&di));
+    {
+        KernelTimer kt("optimal_kernel", s);
+        optimal_kernel<<<ceil_div_u(n_points, kOptThreads), kOptThreads, 0, s>>>(a);
+    }
     count_launch();
-    return check_launch("optimal_kernel");
+    PGEOF_TRY(check_launch("optimal_kernel"));
+    KernelTimer kt("optimal_exact_kernel", s);
+    optimal_exact_kernel<<<std::min<unsigned>(ceil_div_u(n_points, 32), (unsigned)di->sm_count * 8), 64, 0, s>>>(a);
+    count_launch();
+    return check_launch("optimal_exact_kernel");
 }
 
 }  // namespace pgeof
