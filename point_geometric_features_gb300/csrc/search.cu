@@ -1253,7 +1253,12 @@ int launch_fast(const GridView<float>& gv, const CloudTable& ct, const SPoint<fl
     // Radius searches (no pilot bounds to save) keep fixed 16-query items:
     // guided items measured no faster there and lengthened the serving
     // stream's p99 (3.4 vs 2.7 ms over 30 s).
-    if (chunk == 0 && mode != MODE_KNN) chunk = 16;
+    // Small searches go by items that give every resident warp about four
+    // (selected features of 20k points: 16-query items 0.36 ms, most of the GPU
+    // idle and every block waiting for its slowest warp; 6 / 3 / 1 queries 0.185 /
+    // 0.146 / 0.136 ms).
+    if (chunk == 0 && mode != MODE_KNN)
+        chunk = (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, m / (4 * (uint64_t)di->sm_count * per_sm * kFastWarps)));
     const uint32_t chunk_max = chunk ? chunk : guided_max;
     const uint32_t chunk_min = chunk ? chunk : std::min(guided_min, guided_max);
     const uint64_t items = ceil_div_u(m, chunk_min);
