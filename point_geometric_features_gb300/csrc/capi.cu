@@ -283,7 +283,13 @@ int selected_on_grid(const GridIndex<T>& grid, const T* xyz, uint64_t n, T radiu
     for (int64_t off = 0; off < n_ids; off += kSelMaxIds) {
         sp.id_offset = (uint32_t)off;
         sp.n_ids = (int)std::min<int64_t>(kSelMaxIds, n_ids - off);
-        for (int t = 0; t < sp.n_ids; ++t) sp.ids[t] = ids[off + t];
+        sp.axis_only = sp.order == 0 ? 1 : 0;
+        for (int t = 0; t < sp.n_ids; ++t) {
+            sp.ids[t] = ids[off + t];
+            if (sp.ids[t] != PGEOF_NORMAL_X && sp.ids[t] != PGEOF_NORMAL_Y && sp.ids[t] != PGEOF_NORMAL_Z &&
+                sp.ids[t] != PGEOF_VERTICALITY)
+                sp.axis_only = 0;
+        }
         PGEOF_TRY(launch_search<T>(grid, grid.pts, grid.cell_start, n, MODE_RADIUS, k_search, radius, so, s));
     }
     return PGEOF_OK;

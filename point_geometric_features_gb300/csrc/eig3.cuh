@@ -437,6 +437,63 @@ __device__ __forceinline__ void eigvals_f32(const Cov<float>& cov, float (&w)[3]
     if (w[1] < w[0]) { t = w[0]; w[0] = w[1]; w[1] = t; }
 }
 
+// ---- float64: the last (principal, ascending order) axis alone, for callers that
+// want nothing else. GB300 runs float64 at 1/64 of the float rate, and a float64
+// Jacobi solve is a chain of ~1,400 dependent operations (~40 us). Here a float
+// Jacobi solve gives the eigenvectors to ~1e-6, and two steps of the iterative
+// refinement of Ogita and Aishima ("Iterative refinement for symmetric eigenvalue
+// decomposition", Japan J. Indust. Appl. Math. 35, 2018) bring the axis x to
+// float64: with r = 1 - x'x, lambda = x'Ax / (1 - r) and e_i = (u_i'Ax - lambda
+// u_i'x) / (lambda - lambda_i) for the other eigenvectors u_i, x <- x + sum u_i e_i
+// + x r / 2. The error is squared (over the gap) each time; the corrections are
+// ~1e-6, so their denominators need float precision only. Against a long-double
+// solve the vectors are off by <= 5e-15 at gaps from 0.03 on, a float64 Jacobi
+// solve's by 1.5e-14. Only the axis's own gap counts: two or three points, whose
+// smaller eigenvalues are rounding noise, have it too.
+//
+// Left to the float64 Jacobi solver (false): relative gaps below kGapRefine (two
+// steps would not do: 6e-8 / gap, squared over the gap twice, is 1e-17 at 0.03),
+// and an axis within 1e-6 of horizontal (its sign is then the solver's own).
+// out.val and the other axes stay unset.
+constexpr float kGapRefine = 0.03f;
+__device__ __forceinline__ bool pca_axis_f64_refine(const Cov<double>& c, Pca<double>& out) {
+    const double top = fmax(fabs(c.xx), fmax(fabs(c.yy), fabs(c.zz)));
+    if (!(top > 1e-30) || !(top < 1e30)) return false;
+    const float inv = 1.0f / (float)top;
+    float a[3][3], v[3][3], w[3];
+    const Cov<float> cf{(float)c.xx * inv, (float)c.xy * inv, (float)c.xz * inv,
+                        (float)c.yy * inv, (float)c.yz * inv, (float)c.zz * inv};
+    load_cov(cf, a);
+    jacobi3<float, true, false>(a, v);
+    w[0] = a[0][0];
+    w[1] = a[1][1];
+    w[2] = a[2][2];
+    sort_ascending(w, v);
+    if (!(w[2] - w[1] >= kGapRefine * w[2]) || !(fabsf(v[2][2]) >= 1e-6f)) return false;
+    const double g02 = (double)(1.0f / ((w[2] - w[0]) * (float)top)), g12 = (double)(1.0f / ((w[2] - w[1]) * (float)top));
+    double u[3], p[3], x[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        u[r] = (double)v[r][0];
+        p[r] = (double)v[r][1];
+        x[r] = (double)v[r][2];
+    }
+    const auto dot = [](const double (&m)[3], const double (&n)[3]) { return fma(m[0], n[0], fma(m[1], n[1], m[2] * n[2])); };
+#pragma unroll
+    for (int step = 0; step < 2; ++step) {
+        const double y[3] = {fma(c.xx, x[0], fma(c.xy, x[1], c.xz * x[2])), fma(c.xy, x[0], fma(c.yy, x[1], c.yz * x[2])),
+                             fma(c.xz, x[0], fma(c.yz, x[1], c.zz * x[2]))};
+        const double r = 1.0 - dot(x, x), d = dot(x, y), l = fma(d, fma(r, r, r), d);
+        const double e0 = fma(l, -dot(u, x), dot(u, y)) * g02, e1 = fma(l, -dot(p, x), dot(p, y)) * g12;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) x[k] += fma(u[k], e0, fma(p[k], e1, 0.5 * x[k] * r));
+    }
+    const double sign = x[2] < 0.0 ? -1.0 : 1.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out.v[k][2] = sign * x[k];
+    return true;
+}
+
 // --------------------------------------------------------------- epilogues
 template <typename T>
 __device__ __forceinline__ T dev_pow(T x, T y);

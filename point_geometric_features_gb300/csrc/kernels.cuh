@@ -165,6 +165,7 @@ struct SelSpec {
     int n_ids = 0;
     int ids[kSelMaxIds] = {};
     int order = 0;
+    int axis_only = 0;             // ascending order and no id that needs an eigenvalue (float64)
     int ring = 1;                  // queries a warp gathers before its lanes solve them together
 };
 // Queries a warp parks before solving them one per lane: up to 32 while the

@@ -422,15 +422,16 @@ __device__ __forceinline__ void emit_row(int mode, uint32_t k, uint32_t n_sel, u
 
 // ------------------------------------------------------------------ fused selected
 template <typename T>
-__device__ __forceinline__ void solve(const Cov<T>& c, int order, Pca<T>& p);
+__device__ __forceinline__ void solve(const Cov<T>& c, const SelSpec<T>& sp, Pca<T>& p);
 template <>
-__device__ __forceinline__ void solve<float>(const Cov<float>& c, int order, Pca<float>& p) {
+__device__ __forceinline__ void solve<float>(const Cov<float>& c, const SelSpec<float>& sp, Pca<float>& p) {
     bool res;
-    pca_solve_f32(c, order, p, res);
+    pca_solve_f32(c, sp.order, p, res);
 }
 template <>
-__device__ __forceinline__ void solve<double>(const Cov<double>& c, int order, Pca<double>& p) {
-    pca_solve_f64<double>(c, order, &p);
+__device__ __forceinline__ void solve<double>(const Cov<double>& c, const SelSpec<double>& sp, Pca<double>& p) {
+    if (sp.axis_only && pca_axis_f64_refine(c, p)) return;
+    pca_solve_f64<double>(c, sp.order, &p);
 }
 
 // A warp's parking area for selected-feature queries: the sorted neighbour
@@ -512,7 +513,7 @@ __device__ __noinline__ void sel_solve(const SelSpec<T>& sp, const uint32_t* idx
     c.yz = O::div(yz, kk);
     c.zz = O::div(zz, kk);
     Pca<T> p;
-    solve<T>(c, sp.order, p);
+    solve<T>(c, sp, p);
     for (int t = 0; t < sp.n_ids; ++t) {
         T v = T(0);
         if (!selected_feature<T>(p, sp.ids[t], v)) v = T(0);
