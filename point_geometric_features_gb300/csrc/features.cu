@@ -11,8 +11,8 @@
 // after that scale's last neighbour -- the value the reference's own sum over
 // the prefix produces -- the second keeps one product accumulator set per
 // scale; the scales' covariances then wait in shared memory and one copy of
-// the eigen solver handles them in turn. Output rows are staged in shared
-// memory and leave the block as one coalesced slab. The few neighbourhoods
+// the eigen solver handles them in turn. A warp's output rows are staged in
+// its shared memory and leave as one coalesced run. The few neighbourhoods
 // whose float eigenvectors are ill-conditioned are queued and solved exactly
 // afterwards by features_exact_kernel.
 #include <algorithm>
@@ -29,6 +29,11 @@ namespace {
 
 constexpr int kFeatThreads = 128;
 constexpr int kMaxScalesPerLaunch = 8;
+constexpr int kSlabLoads = 8;  // index loads in flight per lane
+// Words between a warp's staged columns: with 33, a lane's column and a row's
+// features are both free of bank conflicts (with 128 a row's features were all
+// in one bank).
+constexpr int kStageCol = 33;
 
 struct FeatArgs {
     const float4* xyz4;
@@ -55,6 +60,7 @@ struct FeatArgs {
     uint32_t row_base;             // this launch covers rows [row_base, row_base + n_points)
     int row_map_input;             // with row_map: row r also reads CSR row row_map[r].idx
     uint32_t slab_words;           // SLAB kernel: index words per warp in shared memory
+    uint32_t warp_words;           // shared memory words per warp (set at the launch)
     // neighbourhoods left to the exact solve: defer[0] counts them, defer[1 ..]
     // holds their output blocks (row * out_scales + scale), whose first six
     // floats carry the covariance until features_exact_kernel replaces them
@@ -131,6 +137,12 @@ __device__ __forceinline__ void gather_row(const uint32_t* nn_all, uint64_t b, u
     for (; j < count; ++j) f(j, gather_nb(xyz4, n_xyz, __ldg(nn + j), flags));
 }
 
+// A word that is read once: not kept in L1, which the gathers need.
+__device__ __forceinline__ uint32_t load_once(const uint32_t* p) {
+    uint32_t v;
+    asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
 
 // gather_row over indices already in shared memory (idx[0 .. count)).
 template <typename F>
@@ -149,11 +161,19 @@ __device__ __forceinline__ void gather_row_slab(const uint32_t* idx, uint32_t co
     for (; j < count; ++j) f(j, gather_nb(xyz4, n_xyz, idx[j], flags));
 }
 
+// What bounds it: the scattered 16-byte gathers, two per neighbour, of which an
+// SM serves 0.9 a cycle from L1 and L2; the solver and the output hide under them.
+//
 // SLAB: the CSR indices of a warp's 32 consecutive rows (one contiguous range
 // of nn when the rows are in CSR order) are read once into shared memory with
-// coalesced loads, and both sweeps take them from there -- instead of each
-// thread reading its own row's indices from global memory in both sweeps.
-// Rows outside the slab (too long, out of order) read global memory.
+// coalesced loads, eight in flight per lane, and both sweeps take them from
+// there -- instead of each thread reading its own row's indices from global
+// memory in both sweeps, which took an L1 request per row for every four
+// neighbours. Rows outside the slab (too long, out of order) read global memory.
+// The staged features take the slab's place after the sweeps. (Keeping the
+// first sweep's coordinates in shared memory as well, so that the second does
+// not gather, left 8 to 16 warps per SM and little L1: 0.77 ms instead of 0.52 on
+// three scales of 50 neighbours.)
 //
 // EXACT_INLINE: neighbourhoods that need the exact solve get it in place.
 // Otherwise they are queued for features_exact_kernel, which keeps the rare
@@ -164,11 +184,12 @@ __device__ __forceinline__ void gather_row_slab(const uint32_t* idx, uint32_t co
 template <int S, bool MULTI, bool SLAB = false, bool EXACT_INLINE = false>
 __device__ __forceinline__ void features_body(const FeatArgs& a) {
     extern __shared__ __align__(16) float smem_f[];
-    float* stage = smem_f;  // kFeatThreads * n_scales * 11, then SLAB: a.slab_words per warp
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
+    // a warp's words: its index slab (SLAB) until both sweeps are done, then its
+    // rows' features, one column per lane, columns of kStageCol words apart
+    float* stage = smem_f + (size_t)(tid >> 5) * a.warp_words;
     const uint32_t i = a.row_base + blockIdx.x * kFeatThreads + tid;
     const int row_w = a.n_scales * 11;
-    for (int f = 0; f < row_w; ++f) stage[f * kFeatThreads + tid] = 0.0f;  // column-major staging
 
     uint32_t flags = 0;
     const bool row_ok = i < a.row_base + a.n_points;
@@ -185,22 +206,50 @@ __device__ __forceinline__ void features_body(const FeatArgs& a) {
     }
     const uint32_t* slab_idx = nullptr;  // this row's indices in shared memory
     if constexpr (SLAB) {
-        const int lane = tid & 31;
         const uint32_t vmask = __ballot_sync(0xffffffffu, row_ok);
         if (vmask && !a.row_map_input) {
             const int last = 31 - __clz(vmask);  // valid rows are a prefix of the warp
             const uint64_t s0 = __shfl_sync(0xffffffffu, b, 0), s1 = __shfl_sync(0xffffffffu, e, last);
-            if (s1 >= s0 && s1 - s0 <= a.slab_words && s1 <= a.nnz) {
-                uint32_t* slab = reinterpret_cast<uint32_t*>(stage + (size_t)kFeatThreads * row_w) +
-                                 (size_t)(tid >> 5) * a.slab_words;
-                for (uint32_t w = lane; w < (uint32_t)(s1 - s0); w += 32) slab[w] = __ldg(a.nn + s0 + w);
+            // rows of one even length are kept an odd number of words apart: end to
+            // end, the lanes' reads meet in a few banks (rows of 32: in one, and two
+            // scales took 0.42 ms)
+            const uint32_t len0 = (uint32_t)__shfl_sync(0xffffffffu, e - b, 0);
+            const bool apart = __all_sync(0xffffffffu, !row_ok || e - b == len0) && len0 > 0 && (len0 & 1u) == 0;
+            if (s1 >= s0 && s1 - s0 + (apart ? 32u : 0u) <= a.slab_words && s1 <= a.nnz) {
+                uint32_t* to = reinterpret_cast<uint32_t*>(stage);
+                const uint32_t* from = a.nn + s0;
+                const uint32_t words = (uint32_t)(s1 - s0);
+                // w / len0 = w * inv >> 22 while w * len0 < 2^22 (w <= 32 * 128 here)
+                const uint32_t inv = apart ? ((1u << 22) + len0 - 1) / len0 : 0u;
+                uint32_t w = lane;
+                for (; w + 32 * (kSlabLoads - 1) < words; w += 32 * kSlabLoads) {
+                    uint32_t v[kSlabLoads];
+#pragma unroll
+                    for (int q = 0; q < kSlabLoads; ++q) v[q] = load_once(from + w + 32 * q);
+#pragma unroll
+                    for (int q = 0; q < kSlabLoads; ++q) to[w + 32 * q + ((w + 32 * q) * inv >> 22)] = v[q];
+                }
+                if (w < words) {
+                    uint32_t v[kSlabLoads - 1];
+#pragma unroll
+                    for (int q = 0; q < kSlabLoads - 1; ++q)
+                        if (w + 32 * q < words) v[q] = load_once(from + w + 32 * q);
+#pragma unroll
+                    for (int q = 0; q < kSlabLoads - 1; ++q)
+                        if (w + 32 * q < words) to[w + 32 * q + ((w + 32 * q) * inv >> 22)] = v[q];
+                }
                 __syncwarp();
-                if (row_ok && b >= s0 && e <= s1 && e >= b) slab_idx = slab + (b - s0);
+                if (row_ok && b >= s0 && e <= s1 && e >= b) slab_idx = to + (b - s0) + (apart ? lane : 0);
             }
         }
     }
+    uint32_t k_nn = 0;
+    uint32_t ks[S];
+    int n_active = 0;
+    float cxx[S], cxy[S], cxz[S], cyy[S], cyz[S], czz[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) cxx[s] = cxy[s] = cxz[s] = cyy[s] = cyz[s] = czz[s] = 0.0f;
     if (row_ok) {
-        uint32_t k_nn = 0;
         if (e < b || e > a.nnz) {
             flags |= ERR_PTR_RANGE;
         } else {
@@ -217,9 +266,6 @@ __device__ __forceinline__ void features_body(const FeatArgs& a) {
             rc.xyz4 = a.xyz4 + a.cloud_off[lo];
             rc.n = (uint32_t)(a.cloud_off[lo + 1] - a.cloud_off[lo]);
         }
-        uint32_t ks[S];
-        int n_active = 0;
-        uint32_t kmax = 0;
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             ks[s] = a.full ? k_nn : a.scales[s];
@@ -229,16 +275,8 @@ __device__ __forceinline__ void features_body(const FeatArgs& a) {
             } else {
                 act = s < a.n_scales && k_nn >= ks[s] && n_active == s;  // break at the first short scale
             }
-            if (act) {
-                n_active = s + 1;
-                kmax = ks[s] > kmax ? ks[s] : kmax;
-            }
+            if (act) n_active = s + 1;
         }
-        // output block of scale s of this row
-        const auto out_block = [&](int s) -> uint64_t {
-            const uint64_t dst = a.row_map ? (uint64_t)a.row_map[i].idx : (uint64_t)i;
-            return dst * (uint64_t)a.out_scales + (uint64_t)(a.scale_offset + s);
-        };
         if (n_active > 0) {
             // neighbours [j0, j1) of the row in order, indices from the slab or global memory
             const auto sweep = [&](uint32_t j0, uint32_t j1, auto&& f) {
@@ -275,9 +313,6 @@ __device__ __forceinline__ void features_body(const FeatArgs& a) {
                 }
             }
             // sweep 2: centred products, sequential sums
-            float cxx[S], cxy[S], cxz[S], cyy[S], cyz[S], czz[S];
-#pragma unroll
-            for (int s = 0; s < S; ++s) cxx[s] = cxy[s] = cxz[s] = cyy[s] = cyz[s] = czz[s] = 0.0f;
             j0 = 0;
 #pragma unroll
             for (int t = 0; t < S; ++t) {
@@ -302,78 +337,91 @@ __device__ __forceinline__ void features_body(const FeatArgs& a) {
                     j0 = j1;
                 }
             }
-            if constexpr (S == 1) {
-                const float kk = (float)ks[0];
-                Cov<float> c;
-                c.xx = FDIV(cxx[0], kk);
-                c.xy = FDIV(cxy[0], kk);
-                c.xz = FDIV(cxz[0], kk);
-                c.yy = FDIV(cyy[0], kk);
-                c.yz = FDIV(cyz[0], kk);
-                c.zz = FDIV(czz[0], kk);
-                float f[11];
-                solve_or_defer<EXACT_INLINE>(a, c, out_block(0), f, flags);
+        }
+    }
+    // output block of scale s of this row
+    const uint64_t dst = a.row_map && row_ok ? (uint64_t)a.row_map[i].idx : (uint64_t)i;
+    const auto out_block = [&](int s) -> uint64_t { return dst * (uint64_t)a.out_scales + (uint64_t)(a.scale_offset + s); };
+    __syncwarp();  // the slab is done with
+    if constexpr (S == 1) {
+        float f[11];
 #pragma unroll
-                for (int q = 0; q < 11; ++q) stage[q * kFeatThreads + tid] = f[q];
-            } else {
-                // park each scale's covariance in its staging slot, then solve the
-                // scales one at a time (one copy of the solver, not S)
+        for (int q = 0; q < 11; ++q) f[q] = 0.0f;
+        if (n_active > 0) {
+            const float kk = (float)ks[0];
+            Cov<float> c;
+            c.xx = FDIV(cxx[0], kk);
+            c.xy = FDIV(cxy[0], kk);
+            c.xz = FDIV(cxz[0], kk);
+            c.yy = FDIV(cyy[0], kk);
+            c.yz = FDIV(cyz[0], kk);
+            c.zz = FDIV(czz[0], kk);
+            solve_or_defer<EXACT_INLINE>(a, c, out_block(0), f, flags);
+        }
 #pragma unroll
-                for (int s = 0; s < S; ++s) {
-                    if (s < n_active) {
-                        const float kk = (float)ks[s];
-                        float* st = stage + (s * 11) * kFeatThreads + tid;
-                        st[0 * kFeatThreads] = FDIV(cxx[s], kk);
-                        st[1 * kFeatThreads] = FDIV(cxy[s], kk);
-                        st[2 * kFeatThreads] = FDIV(cxz[s], kk);
-                        st[3 * kFeatThreads] = FDIV(cyy[s], kk);
-                        st[4 * kFeatThreads] = FDIV(cyz[s], kk);
-                        st[5 * kFeatThreads] = FDIV(czz[s], kk);
-                    }
-                }
-#pragma unroll 1
-                for (int s = 0; s < n_active; ++s) {
-                    float* st = stage + (s * 11) * kFeatThreads + tid;
-                    Cov<float> c;
-                    c.xx = st[0 * kFeatThreads];
-                    c.xy = st[1 * kFeatThreads];
-                    c.xz = st[2 * kFeatThreads];
-                    c.yy = st[3 * kFeatThreads];
-                    c.yz = st[4 * kFeatThreads];
-                    c.zz = st[5 * kFeatThreads];
-                    float f[11];
-                    solve_or_defer<EXACT_INLINE>(a, c, out_block(s), f, flags);
+        for (int q = 0; q < 11; ++q) stage[q * kStageCol + lane] = f[q];
+    } else {
+        // park each scale's covariance in its staging slot, then solve the
+        // scales one at a time (one copy of the solver, not S)
 #pragma unroll
-                    for (int q = 0; q < 11; ++q) st[q * kFeatThreads] = f[q];
-                }
+        for (int s = 0; s < S; ++s) {
+            if (s < n_active) {
+                const float kk = (float)ks[s];
+                float* st = stage + (s * 11) * kStageCol + lane;
+                st[0 * kStageCol] = FDIV(cxx[s], kk);
+                st[1 * kStageCol] = FDIV(cxy[s], kk);
+                st[2 * kStageCol] = FDIV(cxz[s], kk);
+                st[3 * kStageCol] = FDIV(cyy[s], kk);
+                st[4 * kStageCol] = FDIV(cyz[s], kk);
+                st[5 * kStageCol] = FDIV(czz[s], kk);
             }
+        }
+#pragma unroll 1
+        for (int s = 0; s < a.n_scales; ++s) {
+            float* st = stage + (s * 11) * kStageCol + lane;
+            float f[11];
+#pragma unroll
+            for (int q = 0; q < 11; ++q) f[q] = 0.0f;
+            if (s < n_active) {
+                Cov<float> c;
+                c.xx = st[0 * kStageCol];
+                c.xy = st[1 * kStageCol];
+                c.xz = st[2 * kStageCol];
+                c.yy = st[3 * kStageCol];
+                c.yz = st[4 * kStageCol];
+                c.zz = st[5 * kStageCol];
+                solve_or_defer<EXACT_INLINE>(a, c, out_block(s), f, flags);
+            }
+#pragma unroll
+            for (int q = 0; q < 11; ++q) st[q * kStageCol] = f[q];
         }
     }
     if (flags) atomicOr(a.err, flags);
-    __syncthreads();
-    // coalesced write-out of the block's rows
-    const uint32_t row0 = a.row_base + blockIdx.x * kFeatThreads;
-    const uint32_t rows = min((uint32_t)kFeatThreads, a.row_base + a.n_points - row0);
-    if (a.row_map) {
-        // rows processed in another order: each row goes to its mapped output row
-        const int out_w = a.out_scales * 11;
-        for (int t = tid; t < (int)rows * row_w; t += kFeatThreads) {
-            const int r = t / row_w, c = t - r * row_w;
-            const uint64_t dst = a.row_map[row0 + r].idx;
-            a.out[dst * out_w + a.scale_offset * 11 + c] = stage[c * kFeatThreads + r];
+    __syncwarp();
+    // the warp's rows leave in runs of row_w consecutive floats each (rows
+    // processed in another order, row_map, go each to their own place)
+    const uint32_t vrows = __ballot_sync(0xffffffffu, row_ok);
+    const int total = __popc(vrows) * row_w;  // (valid rows are a prefix of the warp)
+    const uint64_t out_w = (uint64_t)a.out_scales * 11;
+    const uint64_t mine = dst * out_w + (uint64_t)a.scale_offset * 11;
+    int r = 0, c = lane;
+    while (c >= row_w) {
+        c -= row_w;
+        ++r;
+    }
+    const bool runs = !a.row_map && a.n_scales == a.out_scales;  // rows side by side: one run of all
+    float* run = a.out + __shfl_sync(0xffffffffu, mine, 0);
+    for (int t0 = 0; t0 < total; t0 += 32) {
+        const uint64_t at = runs ? 0 : __shfl_sync(0xffffffffu, mine, r & 31);
+        if (t0 + lane < total) {
+            const float v = stage[c * kStageCol + r];
+            if (runs) run[t0 + lane] = v;
+            else a.out[at + c] = v;
         }
-    } else if (a.n_scales == a.out_scales) {
-        float* dst = a.out + (uint64_t)row0 * row_w;
-        const int total = rows * row_w;
-        for (int t = tid; t < total; t += kFeatThreads) {
-            const int r = t / row_w, c = t - r * row_w;
-            dst[t] = stage[c * kFeatThreads + r];
-        }
-    } else {
-        const int out_w = a.out_scales * 11;
-        for (int t = tid; t < (int)rows * row_w; t += kFeatThreads) {
-            const int r = t / row_w, c = t - r * row_w;
-            a.out[(uint64_t)(row0 + r) * out_w + a.scale_offset * 11 + c] = stage[c * kFeatThreads + r];
+        c += 32;
+        while (c >= row_w) {
+            c -= row_w;
+            ++r;
         }
     }
 }
@@ -383,15 +431,13 @@ __global__ void __launch_bounds__(kFeatThreads) features_kernel(const __grid_con
     features_body<S, MULTI, SLAB, EXACT_INLINE>(a);
 }
 
-// The 3-scale pass (compute_features_multiscale with three scales, the
-// 1M-point benchmark's case) compiled for 8 resident blocks per SM: 64
-// registers and a 44-byte spill instead of 76 registers and 6 blocks (0.607 ->
-// 0.591 ms on the 1M-point scene).
-template <bool MULTI>
+// The 3-scale pass compiled for 8 resident blocks per SM: 64 registers and a
+// small spill instead of 76 registers and 6 blocks (1M-point scene, 50
+// neighbours: 0.52 and 0.54 ms).
+template <bool MULTI, bool SLAB>
 __global__ void __launch_bounds__(kFeatThreads, 8) features3_kernel(const __grid_constant__ FeatArgs a) {
-    features_body<3, MULTI, false, false>(a);
+    features_body<3, MULTI, SLAB, false>(a);
 }
-
 
 // Coordinates of each CSR row's first neighbour (point 0's for an empty or
 // invalid row): the key by which rows are ordered in space.
@@ -872,8 +918,7 @@ int pad_xyz(const float* xyz, uint64_t n, float4* out, cudaStream_t s) {
     return check_launch("pad_xyz_kernel");
 }
 
-// Index slabs (SLAB kernel) for single-scale passes; PGEOF_FEATURE_SLAB=0
-// turns them off.
+// Index slabs (SLAB kernel); PGEOF_FEATURE_SLAB=0 turns them off.
 bool use_index_slab() {
     static const bool v = [] {
         const char* e = getenv("PGEOF_FEATURE_SLAB");
@@ -883,8 +928,9 @@ bool use_index_slab() {
 }
 
 template <int S>
-static int launch_features_s(const FeatArgs& a, cudaStream_t s) {
-    const size_t stage_bytes = (size_t)kFeatThreads * a.n_scales * 11 * sizeof(float);
+static int launch_features_s(FeatArgs& a, cudaStream_t s) {
+    const uint32_t stage_words = (uint32_t)a.n_scales * 11 * kStageCol;
+    a.warp_words = (std::max(a.slab_words, stage_words) + 3) / 4 * 4;
     const unsigned blocks = ceil_div_u(a.n_points, kFeatThreads);
     KernelTimer kt("features_kernel", s);
     const bool slab = a.slab_words > 0;
@@ -892,9 +938,10 @@ static int launch_features_s(const FeatArgs& a, cudaStream_t s) {
     Kern kern = slab ? (a.n_clouds > 0 ? features_kernel<S, true, true> : features_kernel<S, false, true>)
                      : (a.n_clouds > 0 ? features_kernel<S, true> : features_kernel<S, false>);
     if constexpr (S == 3) {
-        if (!slab) kern = a.n_clouds > 0 ? features3_kernel<true> : features3_kernel<false>;
+        kern = slab ? (a.n_clouds > 0 ? features3_kernel<true, true> : features3_kernel<false, true>)
+                    : (a.n_clouds > 0 ? features3_kernel<true, false> : features3_kernel<false, false>);
     }
-    const size_t smem = stage_bytes + (slab ? (size_t)(kFeatThreads / 32) * a.slab_words * sizeof(uint32_t) : 0);
+    const size_t smem = (size_t)(kFeatThreads / 32) * a.warp_words * sizeof(uint32_t);
     PGEOF_TRY(cap_smem_carveout((const void*)kern, kFeatThreads, (int)smem));
     kern<<<blocks, kFeatThreads, smem, s>>>(a);
     count_launch();
@@ -952,32 +999,43 @@ int launch_features(const float4* xyz4, uint64_t n_xyz, const uint32_t* nn, uint
     return launch_features_exact(out, defer, cap, resolved, s);
 }
 
+// Words of a warp's index slab, 0 for none. It holds rows of the average length
+// (warps whose rows run longer read global memory), each one word further apart
+// if that is even; more words than the rows need would cost resident blocks, and
+// beyond 128 neighbours so would the slab itself. Without and with it, on the
+// 1M-point scene: k = 50 0.437 and 0.376 ms, two scales of 32 neighbours 0.317
+// and 0.284, three of 50 0.571 and 0.521, four of 50 0.737 and 0.568. Several
+// scales of fewer rows than one block per SM go without: there the time is one
+// warp's chain of loads, to which the slab adds its own (5848 rows, two scales:
+// 0.019 and 0.022 ms); the full pass of so few rows takes the same either way.
+static uint32_t index_slab_words(const FeatArgs& a, uint64_t nnz, uint32_t uniform_k, int sm_count) {
+    const uint64_t k = uniform_k ? uniform_k : (nnz + a.n_points - 1) / a.n_points;
+    if (!a.full && a.n_points < (uint32_t)sm_count * kFeatThreads) return 0;
+    if (!use_index_slab() || a.row_map_input || k < 1 || k > 128) return 0;
+    return 32u * ((uint32_t)k | 1u) + 4u;
+}
+
 static int launch_features_impl(FeatArgs& a, uint64_t n_points, bool full, uint64_t k_min, const uint32_t* scales,
                                 int n_scales, uint64_t nnz, uint32_t uniform_k, cudaStream_t s) {
+    const DeviceInfo* di;
+    PGEOF_TRY(current_device_info(&di));
     if (full) {
         a.full = 1;
         a.k_min = (uint32_t)std::min<uint64_t>(k_min, 0xffffffffull);
         a.n_scales = 1;
         a.out_scales = 1;
         a.scale_offset = 0;
-        // Index slab sized for the average row (warps whose rows run longer
-        // read global memory). Single-scale passes only: on the 1M-point scene
-        // it takes the k = 50 compute_features pass from 0.437 to 0.388 ms and
-        // k = 20 from 0.172 to 0.171 ms, but the 3-scale pass from 0.607 to
-        // 0.613 ms. A larger slab than the rows need costs resident blocks
-        // (k = 50 rows in a 64-neighbour slab: 0.399 ms).
-        const uint64_t ks = uniform_k ? uniform_k : (nnz + n_points - 1) / n_points;
-        a.slab_words = use_index_slab() && !a.row_map_input && ks >= 1 && ks <= 128 ? 32u * (uint32_t)ks + 4u : 0u;
+        a.slab_words = index_slab_words(a, nnz, uniform_k, di->sm_count);
         return launch_features_s<1>(a, s);
     }
     a.full = 0;
     a.out_scales = n_scales;
+    a.slab_words = index_slab_words(a, nnz, uniform_k, di->sm_count);
     for (int s0 = 0; s0 < n_scales; s0 += kMaxScalesPerLaunch) {
         const int cnt = std::min(kMaxScalesPerLaunch, n_scales - s0);
         a.n_scales = cnt;
         a.scale_offset = s0;
         for (int q = 0; q < cnt; ++q) a.scales[q] = scales[s0 + q];
-        a.slab_words = 0;
         int st;
         if (cnt == 1) st = launch_features_s<1>(a, s);
         else if (cnt == 2) st = launch_features_s<2>(a, s);
@@ -1166,7 +1224,8 @@ extern "C" int pgeof_compute_features_f32_noalloc(const float* xyz, int64_t n_xy
     a.order = eig_order();
     a.out = features;
     a.err = err;
-    const size_t smem = (size_t)kFeatThreads * 11 * sizeof(float);
+    a.warp_words = 11 * kStageCol + 1;  // (a multiple of 4)
+    const size_t smem = (size_t)(kFeatThreads / 32) * a.warp_words * sizeof(float);
     features_kernel<1, false, false, true><<<ceil_div_u((uint64_t)n_points, kFeatThreads), kFeatThreads, smem, s>>>(a);
     count_launch();
     return check_launch("features_kernel (noalloc)");
