@@ -824,17 +824,23 @@ __global__ void __launch_bounds__(kOptThreads, 12) optimal_kernel(const __grid_c
     }
 }
 
-// The rows optimal_kernel queued, two lanes per row: exact eigentropies of the
-// near-tied sizes (of every size where they found no room), every other size
-// each, and an exact solve of the winner where its eigen-gap is small. A float64
-// solve is a ~40 us chain of dependent operations; the queue's solves run side
-// by side instead of holding up one warp in eight (4M rows: 0.77 ms inside
-// optimal_kernel, 0.23 ms with one lane per row).
+// The rows optimal_kernel queued, 2 to 16 lanes per row: exact eigentropies of the
+// near-tied sizes (of every size where they found no room), dealt out to the
+// lanes, which solve together, and an exact solve of the winner where its eigen-gap
+// is small. What bounds it: a float64 solve is a ~40 us chain of dependent
+// operations, so a row's few solves run side by side, and the queue's do instead of
+// holding up one warp in eight of optimal_kernel (4M rows: 0.77 ms there, 0.23 ms
+// here with one lane per row, 0.15 ms now; 17k rows: 0.07 ms, and 0.145 with two
+// lanes solving in turn). More lanes only where rows are few: a long queue is bound
+// by the float64 pipe (4M rows at kExactLanes = 64: 0.26 ms).
+constexpr uint32_t kExactLanes = 16;  // per block
 __global__ void __launch_bounds__(64) optimal_exact_kernel(const __grid_constant__ OptArgs a) {
-    const uint32_t n = a.queue[0], half = threadIdx.x & 1u;
-    const uint32_t step = gridDim.x * (blockDim.x / 2);
-    for (uint32_t q0 = blockIdx.x * (blockDim.x / 2); q0 < n; q0 += step) {
-        const uint32_t q = q0 + threadIdx.x / 2;
+    const uint32_t n = a.queue[0];
+    uint32_t lanes = 16;  // per row
+    while (lanes > 2 && (uint64_t)n * lanes > (uint64_t)gridDim.x * kExactLanes) lanes /= 2;
+    const uint32_t part = threadIdx.x & (lanes - 1), rows = blockDim.x / lanes;
+    for (uint32_t q0 = blockIdx.x * rows; q0 < n; q0 += gridDim.x * rows) {
+        const uint32_t q = q0 + threadIdx.x / lanes;
         const bool valid = q < n;
         const uint32_t i = a.queue[1 + (valid ? q : q0)];
         float* out = a.out + (uint64_t)i * 12;
@@ -847,9 +853,7 @@ __global__ void __launch_bounds__(64) optimal_exact_kernel(const __grid_constant
         if (cands == 1) {
             k_opt = __float_as_uint(out[1]);
         } else if (cands > 1) {
-            uint32_t turn = 0;
             const auto eval = [&](uint32_t k) {
-                if ((turn++ & 1u) != half) return;
                 const float ent = exact_eigentropy(a, b, k, flags);
                 ++n_exact;
                 if (k_opt == 0xffffffffu || ent < best) {
@@ -858,12 +862,14 @@ __global__ void __launch_bounds__(64) optimal_exact_kernel(const __grid_constant
                 }
             };
             if (cands <= kOptCands) {
-                for (int t = 0; t < cands; ++t) eval(__float_as_uint(out[1 + t]));
+                for (int t = (int)part; t < cands; t += (int)lanes) eval(__float_as_uint(out[1 + t]));
             } else if (sizes.count() > kOptSizes) {
+                uint32_t turn = 0;
                 for (uint32_t k = 1; k <= k_nn; ++k)
-                    if (sizes.take(k)) eval(k);
+                    if (sizes.take(k) && (turn++ & (lanes - 1)) == part) eval(k);
             } else {
                 // the scan again for its minimum, then once more for the sizes near it
+                uint32_t turn = 0;
                 float low = INFINITY;
                 for (int pass = 0; pass < 2; ++pass) {
                     Moments m;
@@ -873,22 +879,26 @@ __global__ void __launch_bounds__(64) optimal_exact_kernel(const __grid_constant
                         if (!each.take(k)) return;
                         const float ent = eigentropy_scan(m.cov(k));
                         if (pass == 0) low = fminf(low, ent);
-                        else if (ent <= low + kTieBand) eval(k);
+                        else if (ent <= low + kTieBand && (turn++ & (lanes - 1)) == part) eval(k);
                     });
                 }
             }
         }
         __syncwarp();
-        // the smaller eigentropy of the two lanes', the smaller size on equality
-        // (a NaN never replaces what came before it)
-        const float other = __shfl_xor_sync(0xffffffffu, best, 1);
-        const uint32_t other_k = __shfl_xor_sync(0xffffffffu, k_opt, 1);
-        const uint32_t first_k = min(k_opt, other_k), last_k = max(k_opt, other_k);
-        const float first = k_opt <= other_k ? best : other, last = k_opt <= other_k ? other : best;
-        k_opt = last_k != 0xffffffffu && last < first ? last_k : first_k;
+        // the smallest eigentropy of the lanes', the smaller size on equality (a
+        // NaN never replaces what came before it)
+        for (uint32_t d = 1; d < lanes; d *= 2) {
+            const float other = __shfl_xor_sync(0xffffffffu, best, d);
+            const uint32_t other_k = __shfl_xor_sync(0xffffffffu, k_opt, d);
+            const uint32_t first_k = min(k_opt, other_k), last_k = max(k_opt, other_k);
+            const float first = k_opt <= other_k ? best : other, last = k_opt <= other_k ? other : best;
+            const bool take = last_k != 0xffffffffu && last < first;
+            k_opt = take ? last_k : first_k;
+            best = take ? last : first;
+        }
         if (flags) atomicOr(a.err, flags);
         if (a.stats && n_exact) atomicAdd(a.stats, (unsigned long long)n_exact);
-        if (valid && half == 0) {
+        if (valid && part == 0) {
             flags = 0;
             if (k_opt == 0xffffffffu) k_opt = sizes.k0;
             Pca<float> p;
@@ -1091,7 +1101,7 @@ int launch_optimal(const float4* xyz4, uint64_t n_xyz, const uint32_t* nn, uint6
     count_launch();
     PGEOF_TRY(check_launch("optimal_kernel"));
     KernelTimer kt("optimal_exact_kernel", s);
-    optimal_exact_kernel<<<std::min<unsigned>(ceil_div_u(n_points, 32), (unsigned)di->sm_count * 8), 64, 0, s>>>(a);
+    optimal_exact_kernel<<<std::min<unsigned>(ceil_div_u(n_points, 4), (unsigned)di->sm_count * 8), 64, 0, s>>>(a);
     count_launch();
     return check_launch("optimal_exact_kernel");
 }
