@@ -277,10 +277,12 @@ __device__ __forceinline__ Smem carve(uint32_t* base, uint32_t k, uint32_t cap, 
 
 // Stages the points of the box's rows that lie within its radius of the
 // queries' box; each warp takes every kWarps-th row, of them the `part`-th of
-// each `parts`. More than `cap` are counted but not kept. (Block-wide between
+// each `parts`. More than `cap` are counted but not kept, and beyond `give_up` the
+// count itself is left incomplete. (Block-wide between
 // barriers; m.ctl[0] is the zeroed count.)
 __device__ __forceinline__ void stage_rows(const GridParams& g, const uint32_t* cell_start, const SPoint<float>* pts,
-                                           const RowBox& b, const Smem& m, uint32_t cap, int part, int parts) {
+                                           const RowBox& b, const Smem& m, uint32_t cap, int part, int parts,
+                                           uint32_t give_up) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const float lim = b.R * b.R * 1.00001f;
     const int rows = (b.rows + parts - 1) / parts;
@@ -303,7 +305,9 @@ __device__ __forceinline__ void stage_rows(const GridParams& g, const uint32_t* 
                 if (!mask) continue;
                 uint32_t at = 0;
                 if (lane == 0) at = atomicAdd(m.ctl, (uint32_t)__popc(mask));
-                at = __shfl_sync(FULL, at, 0) + __popc(mask & ((1u << lane) - 1u));
+                at = __shfl_sync(FULL, at, 0);
+                if (at > give_up) return;
+                at += __popc(mask & ((1u << lane) - 1u));
                 if (near && at < cap) {
                     m.x[at] = p.x;
                     m.y[at] = p.y;
@@ -328,7 +332,7 @@ __device__ __forceinline__ bool restage(const GridParams& g, const uint32_t* cel
     if (threadIdx.x == 0) m.ctl[0] = 0;
     clear_stage(m, stage);
     __syncthreads();
-    stage_rows(g, cell_start, pts, b, m, stage, part, parts);
+    stage_rows(g, cell_start, pts, b, m, stage, part, parts, 0xffffffffu);
     __syncthreads();
     n = m.ctl[0];
     if (n <= stage) return true;
@@ -650,6 +654,13 @@ __global__ void __launch_bounds__(32 * kWarps, 6) group_search_kernel(const __gr
                 uint32_t n = 0, n_take = 0, found = 0, lim = 0;
                 int parts = 1;
                 float too_small = 0.0f;  // a radius known to be short
+                // A radius carried from a sparse place may take in a whole dense
+                // one; counted to the end, a few such groups took 1 to 3 million
+                // cycles each and were the kernel's tail (256 scenes: 9.9 -> 7.4
+                // ms; 33 scenes, k = 20: 2.8 -> 1.1 ms; 2 x, 4 x and 8 x alike).
+                // A radius search cannot shrink: it is given up where its 64
+                // parts could not hold it.
+                const uint32_t give_up = a.stage * (RADIUS ? 64u : 4u);
                 for (int attempt = 0; attempt < 4; ++attempt) {
                     ok = false;
                     set_radius(g, b, R);
@@ -662,13 +673,14 @@ __global__ void __launch_bounds__(32 * kWarps, 6) group_search_kernel(const __gr
                         reinterpret_cast<uint4*>(m.hist)[t * 32 * kWarps + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
                     __syncthreads();
                     parts = 1;
-                    stage_rows(g, cell_start, a.pts, b, m, a.stage, 0, 1);
+                    stage_rows(g, cell_start, a.pts, b, m, a.stage, 0, 1, give_up);
                     __syncthreads();
                     n = m.ctl[0];
                     if (n > a.stage) {
                         // too many: a smaller radius, unless that would be short;
                         // otherwise the rows in several parts
-                        const float less = R * 0.95f * cbrtf((float)a.stage / (float)n);
+                        float less = R * 0.95f * cbrtf((float)a.stage / (float)n);
+                        if (!RADIUS && n > give_up) less = fminf(less, a.first * g.h);
                         if (!RADIUS && attempt < 2 && less > too_small * 1.02f) {
                             R = less;
                             continue;
