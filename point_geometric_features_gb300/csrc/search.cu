@@ -1093,9 +1093,9 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
     if constexpr (SEL) sel_flush_block<float>(a.sel, rg, ring_base, kFastWarps);
 }
 
-template <bool MULTI, bool SEL = false>
+template <bool SEL>
 __global__ void __launch_bounds__(kFastWarps * 32) fast_search_kernel(const __grid_constant__ FastArgs a) {
-    fast_search_body<MULTI, SEL>(a);
+    fast_search_body<false, SEL>(a);
 }
 
 // The single-cloud kNN pass, compiled for 9 resident blocks per SM (56
@@ -1103,6 +1103,13 @@ __global__ void __launch_bounds__(kFastWarps * 32) fast_search_kernel(const __gr
 // ms); the radius pass keeps its natural allocation.
 __global__ void __launch_bounds__(kFastWarps * 32, 9) fast_knn_kernel(const __grid_constant__ FastArgs a) {
     fast_search_body<false, false>(a);
+}
+
+// Several clouds, 7 resident blocks per SM: 72 registers as without the bound, but
+// no spill (leftovers of 256 scenes, k = 32: unbound / 6 / 7 / 8 / 9 blocks 5.67 /
+// 6.07 / 5.46 / 5.75 / 5.74 ms).
+__global__ void __launch_bounds__(kFastWarps * 32, 7) fast_batch_kernel(const __grid_constant__ FastArgs a) {
+    fast_search_body<true, false>(a);
 }
 
 template <typename T>
@@ -1233,8 +1240,8 @@ int launch_fast(const GridView<float>& gv, const CloudTable& ct, const SPoint<fl
     const int ring_smem = out.sel ? (int)(kFastWarps * sel_ring_bytes(out.sel->max_knn, out.sel->ring)) : 0;
     const int smem =
         (int)(kFastWarps * (sizeof(FastWarpSmem) + (size_t)(cap + cap_sorted) * sizeof(uint64_t))) + ring_smem;
-    auto kern = out.sel ? fast_search_kernel<false, true>
-                        : (ct.n ? fast_search_kernel<true>
+    auto kern = out.sel ? fast_search_kernel<true>
+                        : (ct.n ? fast_batch_kernel
                                 : (mode == MODE_KNN ? fast_knn_kernel : fast_search_kernel<false>));
     int per_sm = 0;
     PGEOF_TRY(kernel_blocks_per_sm((const void*)kern, kFastWarps * 32, smem, &per_sm));
