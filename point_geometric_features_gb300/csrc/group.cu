@@ -56,6 +56,13 @@ constexpr int kBinsPerWarp = kBins / kWarps;
 // at k = 50; gaps 0.75 / 1.5: 1.297 / 1.328 ms at k = 50.)
 constexpr float kGroupGap = 0.75f;
 constexpr float kGroupWidth = 2.0f;
+// A radius search's edge is at most the radius, which in sparse clouds leaves a
+// cell few points; its R does not grow with the group's own k-th distances either,
+// so wider groups only bring more company (2.6M points, 33 per square metre, radius
+// 0.56 / 64: one query per warp 2.35 ms, gap / width 0.75 / 2 2.42, 1 / 4 2.19, 1 / 6
+// 2.18, 1.5 / 8 2.16; 400k points, 0.4 / 30: 0.41, 0.46, 0.40, 0.39, 0.38; dense
+// clouds cut their runs at 32 members first: 4M points, 0.5 / 64 4.39, 4.40, 4.40, 4.41).
+constexpr float kRadiusGap = 1.0f, kRadiusWidth = 6.0f;
 // (1.06 / 1.1: 1.190 / 1.211 ms on the scene, k = 50, 1.196 / 1.211 ms on
 // a uniform cube.)
 constexpr float kGroupSlack = 1.07f;  // R over the largest k-th distance of the group before
@@ -930,8 +937,8 @@ int launch_group_search(const GroupSearch& q, const SearchOut<float>& out, cudaS
     sp.ct = q.ct;
     sp.queries = q.queries;
     sp.m = q.m;
-    sp.gap = kGroupGap;
-    sp.width = kGroupWidth;
+    sp.gap = rad ? kRadiusGap : kGroupGap;
+    sp.width = rad ? kRadiusWidth : kGroupWidth;
     sp.groups = static_cast<Group*>(q.groups);
     sp.group_count = q.counters + 1;
     sp.rest = q.rest;
