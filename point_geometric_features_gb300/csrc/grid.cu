@@ -37,7 +37,7 @@ static inline float ord_decode(uint32_t k) {
 }
 
 template <typename T>
-__global__ void bbox_kernel(const T* __restrict__ xyz, uint64_t n, uint32_t* out6) {
+__global__ void bbox_kernel(const T* __restrict__ xyz, uint64_t n, uint32_t* out6) {  // (out6 zeroed; see box_min)
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
 #pragma unroll
@@ -51,11 +51,13 @@ __global__ void bbox_kernel(const T* __restrict__ xyz, uint64_t n, uint32_t* out
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            atomicMin(out6 + a, ord_key(mn[a]));
+            atomicMax(out6 + a, ~ord_key(mn[a]));
             atomicMax(out6 + 3 + a, ord_key(mx[a]));
         }
     }
 }
+// The smallest coordinate is kept complemented, so that zeros start both ends.
+float box_min(uint32_t key) { return ord_decode(~key); }
 
 template <typename T>
 __device__ __forceinline__ uint32_t cell_of(const GridParams& g, T x, T y, T z) {
@@ -228,13 +230,6 @@ unsigned grid_blocks(uint64_t n, int threads) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u(n, threads), cap));
 }
 
-int exclusive_scan(const uint32_t* in, uint32_t G, uint32_t* out, cudaStream_t s) {
-    const uint32_t nb = ceil_div_u(G, kScanTile);
-    Scratch part;
-    PGEOF_TRY(part.alloc((size_t)nb * sizeof(uint32_t), s));
-    return exclusive_scan_into(in, G, out, part.as<uint32_t>(), s);
-}
-
 struct HostBox {
     float mn[3], mx[3];
 };
@@ -366,20 +361,29 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
     Scratch misc;
     PGEOF_TRY(misc.alloc(64, s));
     uint32_t* box = misc.as<uint32_t>();
-    PGEOF_CUDA_TRY(cudaMemsetAsync(box, 0xff, 3 * sizeof(uint32_t), s));
-    PGEOF_CUDA_TRY(cudaMemsetAsync(box + 3, 0, 3 * sizeof(uint32_t), s));
+    PGEOF_CUDA_TRY(cudaMemsetAsync(box, 0, 6 * sizeof(uint32_t), s));
     {
         KernelTimer kt("bbox_kernel", s);
         bbox_kernel<T><<<grid_blocks(n, 256), 256, 0, s>>>(xyz, n, box);
     }
     count_launch();
     PGEOF_TRY(check_launch("bbox_kernel"));
+    // Buffers of a size known already: in small clouds taken before the wait, after
+    // which the GPU idles until the next launch (10k points: 80 -> 76 us a search);
+    // in large ones after the trials' scratch has gone.
+    Scratch cell_rank;
+    const auto point_buffers = [&]() -> int {
+        PGEOF_TRY(out.pts_mem.alloc((size_t)n * sizeof(SPoint<T>), s));
+        return cell_rank.alloc(2 * (size_t)n * sizeof(uint32_t), s);
+    };
+    const bool early = n <= (1u << 20);
+    if (early) PGEOF_TRY(point_buffers());
     uint32_t hb[6];
     PGEOF_CUDA_TRY(cudaMemcpyAsync(hb, box, sizeof(hb), cudaMemcpyDeviceToHost, s));
     PGEOF_CUDA_TRY(cudaStreamSynchronize(s));
     HostBox b;
     for (int a = 0; a < 3; ++a) {
-        b.mn[a] = ord_decode(hb[a]);
+        b.mn[a] = box_min(hb[a]);
         b.mx[a] = ord_decode(hb[3 + a]);
         if (!(b.mn[a] <= b.mx[a]) || !std::isfinite(b.mn[a]) || !std::isfinite(b.mx[a]))
             return fail(PGEOF_ERR_INVALID_ARGUMENT, "point coordinates must be finite");
@@ -478,26 +482,24 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
     }
     out.g = g;
     // 3. counting sort into cells
+    if (!early) PGEOF_TRY(point_buffers());
     PGEOF_TRY(out.cell_mem.alloc(((size_t)g.n_cells + 1) * sizeof(uint32_t), s));
-    PGEOF_TRY(out.pts_mem.alloc((size_t)n * sizeof(SPoint<T>), s));
     out.cell_start = out.cell_mem.template as<uint32_t>();
     out.pts = out.pts_mem.template as<SPoint<T>>();
-    Scratch counts, cell, rank;
-    PGEOF_TRY(counts.alloc((size_t)g.n_cells * sizeof(uint32_t), s));
-    PGEOF_TRY(cell.alloc((size_t)n * sizeof(uint32_t), s));
-    PGEOF_TRY(rank.alloc((size_t)n * sizeof(uint32_t), s));
+    uint32_t* const cell = cell_rank.as<uint32_t>();
+    uint32_t* const rank = cell + n;
+    Scratch counts;  // and the scan's partials
+    PGEOF_TRY(counts.alloc(((size_t)g.n_cells + ceil_div_u(g.n_cells, kScanTile)) * sizeof(uint32_t), s));
     PGEOF_CUDA_TRY(cudaMemsetAsync(counts.p, 0, (size_t)g.n_cells * sizeof(uint32_t), s));
     {
         KernelTimer kt("hist_kernel", s);
-        hist_kernel<T><<<grid_blocks(n, 256), 256, 0, s>>>(xyz, n, g, counts.as<uint32_t>(), cell.as<uint32_t>(),
-                                                            rank.as<uint32_t>());
+        hist_kernel<T><<<grid_blocks(n, 256), 256, 0, s>>>(xyz, n, g, counts.as<uint32_t>(), cell, rank);
     }
     count_launch();
     PGEOF_TRY(check_launch("hist_kernel"));
-    PGEOF_TRY(exclusive_scan(counts.as<uint32_t>(), g.n_cells, out.cell_start, s));
+    PGEOF_TRY(exclusive_scan_into(counts.as<uint32_t>(), g.n_cells, out.cell_start, counts.as<uint32_t>() + g.n_cells, s));
     KernelTimer kt("scatter_kernel", s);
-    scatter_kernel<T><<<grid_blocks(n, 256), 256, 0, s>>>(xyz, n, out.cell_start, cell.as<uint32_t>(),
-                                                           rank.as<uint32_t>(), out.pts);
+    scatter_kernel<T><<<grid_blocks(n, 256), 256, 0, s>>>(xyz, n, out.cell_start, cell, rank, out.pts);
     count_launch();
     return check_launch("scatter_kernel");
 }
@@ -508,23 +510,24 @@ int sort_queries(const T* q, uint64_t m, const GridParams& g, Scratch& out_mem, 
     *out = nullptr;
     if (m == 0) return PGEOF_OK;
     PGEOF_TRY(out_mem.alloc((size_t)m * sizeof(SPoint<T>), s));
-    Scratch counts, cell, rank;
-    PGEOF_TRY(counts.alloc((size_t)g.n_cells * sizeof(uint32_t), s));
+    // counts, the scan's partials, then cell and rank of every query
+    Scratch mem;
+    const size_t head = (size_t)g.n_cells + ceil_div_u(g.n_cells, kScanTile);
+    PGEOF_TRY(mem.alloc((head + 2 * (size_t)m) * sizeof(uint32_t), s));
     PGEOF_TRY(start.alloc(((size_t)g.n_cells + 1) * sizeof(uint32_t), s));
-    PGEOF_TRY(cell.alloc((size_t)m * sizeof(uint32_t), s));
-    PGEOF_TRY(rank.alloc((size_t)m * sizeof(uint32_t), s));
-    PGEOF_CUDA_TRY(cudaMemsetAsync(counts.p, 0, (size_t)g.n_cells * sizeof(uint32_t), s));
+    uint32_t* const counts = mem.as<uint32_t>();
+    uint32_t* const cell = counts + head;
+    uint32_t* const rank = cell + m;
+    PGEOF_CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)g.n_cells * sizeof(uint32_t), s));
     {
         KernelTimer kt("query_hist_kernel", s);
-        hist_kernel<T><<<grid_blocks(m, 256), 256, 0, s>>>(q, m, g, counts.as<uint32_t>(), cell.as<uint32_t>(),
-                                                            rank.as<uint32_t>());
+        hist_kernel<T><<<grid_blocks(m, 256), 256, 0, s>>>(q, m, g, counts, cell, rank);
     }
     count_launch();
     PGEOF_TRY(check_launch("hist_kernel(queries)"));
-    PGEOF_TRY(exclusive_scan(counts.as<uint32_t>(), g.n_cells, start.as<uint32_t>(), s));
+    PGEOF_TRY(exclusive_scan_into(counts, g.n_cells, start.as<uint32_t>(), counts + g.n_cells, s));
     KernelTimer kt("query_scatter_kernel", s);
-    scatter_kernel<T><<<grid_blocks(m, 256), 256, 0, s>>>(q, m, start.as<uint32_t>(), cell.as<uint32_t>(),
-                                                           rank.as<uint32_t>(), out_mem.as<SPoint<T>>());
+    scatter_kernel<T><<<grid_blocks(m, 256), 256, 0, s>>>(q, m, start.as<uint32_t>(), cell, rank, out_mem.as<SPoint<T>>());
     count_launch();
     *out = out_mem.as<SPoint<T>>();
     return check_launch("scatter_kernel(queries)");
