@@ -30,6 +30,7 @@ namespace {
 constexpr int kFeatThreads = 128;
 constexpr int kMaxScalesPerLaunch = 8;
 constexpr int kSlabLoads = 8;  // index loads in flight per lane
+constexpr uint32_t kApartMax = 128;  // longest rows kept an odd number of words apart in the slab
 // Words between a warp's staged columns: with 33, a lane's column and a row's
 // features are both free of bank conflicts (with 128 a row's features were all
 // in one bank).
@@ -214,12 +215,15 @@ __device__ __forceinline__ void features_body(const FeatArgs& a) {
             // end, the lanes' reads meet in a few banks (rows of 32: in one, and two
             // scales took 0.42 ms)
             const uint32_t len0 = (uint32_t)__shfl_sync(0xffffffffu, e - b, 0);
-            const bool apart = __all_sync(0xffffffffu, !row_ok || e - b == len0) && len0 > 0 && (len0 & 1u) == 0;
+            // (longer ones end to end: the last warp of a pass may hold a few rows of thousands,
+            // for which the quotient below is not exact)
+            const bool apart = __all_sync(0xffffffffu, !row_ok || e - b == len0) && len0 > 0 && len0 <= kApartMax &&
+                               (len0 & 1u) == 0;
             if (s1 >= s0 && s1 - s0 + (apart ? 32u : 0u) <= a.slab_words && s1 <= a.nnz) {
                 uint32_t* to = reinterpret_cast<uint32_t*>(stage);
                 const uint32_t* from = a.nn + s0;
                 const uint32_t words = (uint32_t)(s1 - s0);
-                // w / len0 = w * inv >> 22 while w * len0 < 2^22 (w <= 32 * 128 here)
+                // w / len0 = w * inv >> 22 while w * len0 < 2^22 (w < 32 * len0, len0 <= kApartMax)
                 const uint32_t inv = apart ? ((1u << 22) + len0 - 1) / len0 : 0u;
                 uint32_t w = lane;
                 for (; w + 32 * (kSlabLoads - 1) < words; w += 32 * kSlabLoads) {
