@@ -515,6 +515,14 @@ int pgeof::kernel_blocks_per_sm(const void* kernel, int threads, int smem, int* 
             lim->limit = smem;
         }
     }
+    // The query counts blocks under the kernel's carveout preference of the moment: a
+    // cap left by a launch of another size would make this one look as if it fitted
+    // under the cap by itself, and then run without it.
+    for (CarveEntry& e : g_carve)
+        if (e.device == dev && e.kernel == kernel && e.carveout != -1) {
+            PGEOF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, -1));
+            e.carveout = -1;
+        }
     int n = 0;
     PGEOF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
     n = std::max(n, 1);
