@@ -1015,17 +1015,32 @@ int launch_features(const float4* xyz4, uint64_t n_xyz, const uint32_t* nn, uint
 
 // Words of a warp's index slab, 0 for none. It holds rows of the average length
 // (warps whose rows run longer read global memory), each one word further apart
-// if that is even; more words than the rows need would cost resident blocks, and
-// beyond 128 neighbours so would the slab itself. Without and with it, on the
-// 1M-point scene: k = 50 0.437 and 0.376 ms, two scales of 32 neighbours 0.317
-// and 0.284, three of 50 0.571 and 0.521, four of 50 0.737 and 0.568. Several
-// scales of fewer rows than one block per SM go without: there the time is one
+// if that is even. `nnz`: the neighbours of the rows of this launch.
+//
+// Up to which length: while its blocks leave warps enough to hide the gathers.
+// Without and with it, 1M-point scene, one scale of 50 / 80 / 100 / 128 neighbours
+// 0.484 and 0.420 / 0.717 and 0.648 / 0.904 and 0.856 ms / (200k points) 0.291 and
+// 0.309; two of 50 / 64 / 80 0.546 and 0.477 / 0.612 and 0.590 / 0.743 and 0.732 (200k
+// points, 64 / 80: 0.178 and 0.184 / 0.203 and 0.214); three of 50 / 60 / 64 / 80 0.639 and
+// 0.572 / 0.689 and 0.659 / 0.669 and 0.682 / 0.805 and 0.838; four of 50 / 80 / 100 0.780 and 0.619 / 0.903 and 0.865 / 1.074 and
+// 1.156.
+//
+// Rows of different lengths fill it badly: half of the warps go without, and all
+// pay for its room. A mean that is no whole number tells them (on kNN rows it
+// is one); they have a slab while it is small. Radius rows of the same scene, mean 19 /
+// 29 / 33 / 52 neighbours, two scales: 0.287 and 0.279 / 0.340 and 0.365 / 0.332 and 0.354 /
+// 0.397 and 0.454 ms; three of mean 19 / 52 0.429 and 0.394 / 0.524 and 0.596.
+//
+// Several scales of fewer rows than one block per SM go without: there the time is one
 // warp's chain of loads, to which the slab adds its own (5848 rows, two scales:
 // 0.019 and 0.022 ms); the full pass of so few rows takes the same either way.
+constexpr uint64_t kSlabRagged = 24;
 static uint32_t index_slab_words(const FeatArgs& a, uint64_t nnz, uint32_t uniform_k, int sm_count) {
     const uint64_t k = uniform_k ? uniform_k : (nnz + a.n_points - 1) / a.n_points;
+    const bool even_rows = uniform_k || nnz % a.n_points == 0;
+    const uint64_t limit = !even_rows ? kSlabRagged : a.out_scales == 1 ? 100 : a.out_scales <= 3 ? 60 : 80;
     if (!a.full && a.n_points < (uint32_t)sm_count * kFeatThreads) return 0;
-    if (!use_index_slab() || a.row_map_input || k < 1 || k > 128) return 0;
+    if (!use_index_slab() || a.row_map_input || k < 1 || k > limit) return 0;
     return 32u * ((uint32_t)k | 1u) + 4u;
 }
 
