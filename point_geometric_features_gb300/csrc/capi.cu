@@ -1076,7 +1076,7 @@ static int host_features(const float* xyz, int64_t n_xyz, const uint32_t* nn, in
             }
             status = launch_features(xyz4.as<float4>(), n_xyz, d_nn.as<uint32_t>(), total, d_ptr.as<uint32_t>(),
                                      r1 - r0, kind == 0, k_min, scales, (int)n_scales, d_out.as<float>(), nullptr, s,
-                                     nullptr, 0, nullptr, 0, r0);
+                                     nullptr, 0, nullptr, 0, r0, false, nullptr, hi - lo);
             if (status != PGEOF_OK) break;
             if (cudaEventRecord(ev[2 + 2 * c], s) != cudaSuccess ||
                 cudaStreamWaitEvent(cout, ev[2 + 2 * c], 0) != cudaSuccess ||

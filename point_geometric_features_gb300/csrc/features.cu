@@ -980,7 +980,7 @@ int launch_features(const float4* xyz4, uint64_t n_xyz, const uint32_t* nn, uint
                     uint64_t n_points, bool full, uint64_t k_min, const uint32_t* scales, int n_scales,
                     float* out, unsigned long long* resolved, cudaStream_t s, const uint64_t* cloud_off,
                     int n_clouds, const SPoint<float>* row_map, uint32_t uniform_k, uint64_t row_base,
-                    bool row_map_input, unsigned long long* defer) {
+                    bool row_map_input, unsigned long long* defer, uint64_t slice_nnz) {
     if (n_points == 0) return PGEOF_OK;
     if (!full && n_scales <= 0) return PGEOF_OK;
     // queue for the exact solves: a count and one slot per output block
@@ -1009,7 +1009,7 @@ int launch_features(const float4* xyz4, uint64_t n_xyz, const uint32_t* nn, uint
     a.order = eig_order();
     a.err = device_error_word();
     a.out = out;
-    PGEOF_TRY(launch_features_impl(a, n_points, full, k_min, scales, n_scales, nnz, uniform_k, s));
+    PGEOF_TRY(launch_features_impl(a, n_points, full, k_min, scales, n_scales, slice_nnz ? slice_nnz : nnz, uniform_k, s));
     return launch_features_exact(out, defer, cap, resolved, s);
 }
 

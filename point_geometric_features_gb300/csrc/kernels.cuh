@@ -15,13 +15,16 @@ int pad_xyz(const float* xyz, uint64_t n, float4* out, cudaStream_t s);
 // row_base: the launch covers rows [row_base, row_base + n_points) of ptr / out.
 // row_map_input: row i also reads CSR row row_map[i].idx (rows processed in the
 // order of row_map, each written to its own output row).
+// slice_nnz: neighbours of these rows, where they are a slice of the CSR's (speed
+// only; 0: all nnz of them).
 template <typename T>
 struct SPoint;
 int launch_features(const float4* xyz4, uint64_t n_xyz, const uint32_t* nn, uint64_t nnz, const uint32_t* ptr,
                     uint64_t n_points, bool full, uint64_t k_min, const uint32_t* scales, int n_scales,
                     float* out, unsigned long long* resolved, cudaStream_t s, const uint64_t* cloud_off = nullptr,
                     int n_clouds = 0, const SPoint<float>* row_map = nullptr, uint32_t uniform_k = 0,
-                    uint64_t row_base = 0, bool row_map_input = false, unsigned long long* defer = nullptr);
+                    uint64_t row_base = 0, bool row_map_input = false, unsigned long long* defer = nullptr,
+                    uint64_t slice_nnz = 0);
 // The three CSR feature passes for a float64 cloud (kind 0 compute_features,
 // 1 multiscale over the HOST array `scales`, 2 optimal); out is float64 with
 // rows of 11, n_scales * 11 or 12 values.
