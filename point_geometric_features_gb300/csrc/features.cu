@@ -491,8 +491,8 @@ __global__ void pad_xyz_kernel(const float* __restrict__ xyz, uint64_t n, float4
 
 // ------------------------------------------------------------------ optimal
 constexpr int kOptThreads = 64;
-constexpr int kOptCands = 8;       // near-tied sizes kept per point
-constexpr uint32_t kOptSizes = 64;  // points with more candidate sizes have all of them evaluated exactly
+constexpr int kOptCands = 11;      // near-tied sizes kept per point: what its output row holds beside their number
+constexpr uint32_t kOptSizes = 64;  // (a bit each) points with more candidate sizes have all of them evaluated exactly
 
 struct OptArgs {
     const float4* xyz4;
@@ -713,6 +713,10 @@ struct Sizes {
         const uint32_t multiples = k_nn / step - k0 / step;  // in (k0, k_nn]
         return 1 + multiples + (k_nn > k0 && k_nn % step != 0);
     }
+    __device__ __forceinline__ uint32_t at(uint32_t t) const {  // the t-th of count()
+        const uint64_t k = ((uint64_t)(k0 / step) + t) * step;
+        return t == 0 ? k0 : (uint32_t)(k < k_nn ? k : k_nn);
+    }
     __device__ __forceinline__ bool take(uint32_t k) {  // (called for k = 1, 2, ...)
         if (k == due) {
             due = step == 1 ? k + 1 : (k / step + 1) * step;
@@ -829,14 +833,15 @@ __global__ void __launch_bounds__(kOptThreads, 12) optimal_kernel(const __grid_c
 }
 
 // The rows optimal_kernel queued, 2 to 16 lanes per row: exact eigentropies of the
-// near-tied sizes (of every size where they found no room), dealt out to the
-// lanes, which solve together, and an exact solve of the winner where its eigen-gap
-// is small. What bounds it: a float64 solve is a ~40 us chain of dependent
+// near-tied sizes (found again by a scan where they had no room; every size of
+// rows with more than kOptSizes), dealt out to the lanes, which solve together, and
+// an exact solve of the winner where its eigen-gap is small. What bounds it: a float64 solve is a ~40 us chain of dependent
 // operations, so a row's few solves run side by side, and the queue's do instead of
 // holding up one warp in eight of optimal_kernel (4M rows: 0.77 ms there, 0.23 ms
 // here with one lane per row, 0.15 ms now; 17k rows: 0.07 ms, and 0.145 with two
-// lanes solving in turn). More lanes only where rows are few: a long queue is bound
-// by the float64 pipe (4M rows at kExactLanes = 64: 0.26 ms).
+// lanes solving in turn; 65 sizes of each of 200k rows 36.7 ms, and 74.2). More lanes
+// only where rows are few: a long queue is bound by the float64 pipe (4M rows at
+// kExactLanes = 64: 0.26 ms).
 constexpr uint32_t kExactLanes = 16;  // per block
 __global__ void __launch_bounds__(64) optimal_exact_kernel(const __grid_constant__ OptArgs a) {
     const uint32_t n = a.queue[0];
@@ -868,24 +873,30 @@ __global__ void __launch_bounds__(64) optimal_exact_kernel(const __grid_constant
             if (cands <= kOptCands) {
                 for (int t = (int)part; t < cands; t += (int)lanes) eval(__float_as_uint(out[1 + t]));
             } else if (sizes.count() > kOptSizes) {
-                uint32_t turn = 0;
-                for (uint32_t k = 1; k <= k_nn; ++k)
-                    if (sizes.take(k) && (turn++ & (lanes - 1)) == part) eval(k);
+                for (uint32_t t = part; t < sizes.count(); t += lanes) eval(sizes.at(t));
             } else {
-                // the scan again for its minimum, then once more for the sizes near it
-                uint32_t turn = 0;
+                // the scan again for its minimum, then once more for the sizes near it, a
+                // bit each; the lane's own are solved after the scan, where the warp's
+                // lanes solve together (solved at their place in it, they waited for one
+                // another: 200k rows of a 0.5 m voxel grid, 64 neighbours, 5.2 ms)
                 float low = INFINITY;
+                uint64_t near = 0, mine = 0;
                 for (int pass = 0; pass < 2; ++pass) {
                     Moments m;
                     Sizes each(a, k_nn);
+                    uint32_t t = 0;
                     offset_row(a, b, k_nn, flags, [&](uint32_t k, float dx, float dy, float dz) {
                         m.add(dx, dy, dz);
                         if (!each.take(k)) return;
                         const float ent = eigentropy_scan(m.cov(k));
                         if (pass == 0) low = fminf(low, ent);
-                        else if (ent <= low + kTieBand && (turn++ & (lanes - 1)) == part) eval(k);
+                        else if (ent <= low + kTieBand) near |= 1ull << t;
+                        ++t;
                     });
                 }
+                for (uint32_t t = 0; near; near &= near - 1, ++t)
+                    if ((t & (lanes - 1)) == part) mine |= near & (0ull - near);
+                for (; mine; mine &= mine - 1) eval(sizes.at((uint32_t)__ffsll((long long)mine) - 1));
             }
         }
         __syncwarp();
