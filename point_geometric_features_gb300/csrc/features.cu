@@ -546,14 +546,42 @@ struct KSum2 {
     }
 };
 
+// The two smaller eigenvalues, about zero and about equal beside the largest one, e2:
+// those of A with its principal axis v taken out, C = A - e2 v v', from the trace of C
+// and the sum of its squares. v is the cross product of two rows of A - e2, scaled to
+// about 1 by `scale`.
+__device__ __noinline__ float2 smaller_two(const Cov<float> c, float e2, float scale) {
+    const bool y = c.yy > c.xx, z = c.zz > fmaxf(c.xx, c.yy);  // the largest diagonal's row is left out
+    const float xx = (c.xx - e2) * scale, yy = (c.yy - e2) * scale, zz = (c.zz - e2) * scale;
+    const float xy = c.xy * scale, xz = c.xz * scale, yz = c.yz * scale;
+    const float ax = z || y ? xx : xy, ay = z || y ? xy : yy, az = z || y ? xz : yz;  // row x, or y
+    const float bx = z ? xy : xz, by = z ? yy : yz, bz = z ? yz : zz;                 // row z, or y
+    const float vx = ay * bz - az * by, vy = az * bx - ax * bz, vz = ax * by - ay * bx;
+    const float n = vx * vx + vy * vy + vz * vz;
+    const float s = n > 1e-30f ? __fdividef(e2, n) : 0.0f;
+    const float dx = c.xx - s * vx * vx, dy = c.yy - s * vy * vy, dz = c.zz - s * vz * vz;
+    const float ex = c.xy - s * vx * vy, ey = c.xz - s * vx * vz, ez = c.yz - s * vy * vz;
+    const float half = 0.5f * (dx + dy + dz), squares = dx * dx + dy * dy + dz * dz + 2.0f * (ex * ex + ey * ey + ez * ez);
+    const float apart = sqrtf(fmaxf(0.5f * squares - half * half, 0.0f));
+    return make_float2(half - apart, half + apart);
+}
+
 // Eigentropy (include/pca.hpp:140-150) of a covariance for ranking candidate
 // sizes: the trigonometric closed form of the eigenvalues (O. K. Smith,
 // "Eigenvalues of a symmetric 3x3 matrix", CACM 4(4), 1961). Every size within
 // kTieBand (3e-5) of the minimum is re-evaluated exactly, so these values need
 // only stay within half the band of the exact ones. The arc cosine is
 // Abramowitz & Stegun 4.4.46 (error <= 2e-8) and the other functions are the
-// hardware's (__cosf: absolute error < 2^-21 on [-pi, pi]; __logf): about 1e-6
-// in the eigentropy.
+// hardware's (__cosf: absolute error < 2^-21 on [-pi, pi]; __logf): ~1e-6 in the
+// eigentropy, with an exact arc cosine as with this one (300k covariances each of
+// planes, volumes, isotropic and mixed points). Where the two smaller eigenvalues
+// nearly meet (r near 1) the arc cosine magnifies r's rounding to 1e-4 of the largest
+// one; where they are next to nothing as well, on a line, that is up to 1.4e-3 in the
+// eigentropy and chose other sizes. There they come from smaller_two (6e-6 at most); the
+// scan of all rows, which has no registers for it (4M rows: 3.38 -> 3.52 ms), asks for
+// no more than `line`, and leaves such rows to optimal_exact_kernel.
+constexpr float kLine = 0.999f;
+constexpr float kThin = 0.02f;
 __device__ __forceinline__ float eigentropy_scan(const Cov<float>& c) {
     const float q = (c.xx + c.yy + c.zz) * (1.0f / 3.0f);
     const float b00 = c.xx - q, b11 = c.yy - q, b22 = c.zz - q;
@@ -578,8 +606,13 @@ __device__ __forceinline__ float eigentropy_scan(const Cov<float>& c) {
     a *= y > 0.0f ? y * rsqrtf(y) : 0.0f;
     const float phi = (r < 0.0f ? 3.14159265f - a : a) * (1.0f / 3.0f);
     const float e2 = q + 2.0f * p * __cosf(phi);
-    const float e0 = q + 2.0f * p * __cosf(phi + 2.0943951023931953f);
-    const float e1 = 3.0f * q - e0 - e2;
+    float e0 = q + 2.0f * p * __cosf(phi + 2.0943951023931953f);
+    float e1 = 3.0f * q - e0 - e2;
+    if (r > kLine && e0 + e1 <= kThin * e2) {
+        const float2 e = smaller_two(c, e2, inv_p);
+        e0 = e.x;
+        e1 = e.y;
+    }
     const float v0 = fmaxf(e0, 0.0f), v1 = fmaxf(e1, 0.0f), v2 = fmaxf(e2, 0.0f);
     const float eps = 1e-3f;
     const float inv = __fdividef(1.0f, v0 + v1 + v2 + eps);

@@ -1,5 +1,5 @@
 """compute_features_optimal where sizes tie or are many (csrc/features.cu): more near-tied
-sizes than a row keeps, more sizes than the scan ranks, rows that are planes,
+sizes than a row keeps, more sizes than the scan ranks, rows that are lines, planes,
 duplicates or a voxel grid. The size found has the smallest float64 eigentropy up to the
 rounding of the float formula (its terms are below 1 and hold ~10 roundings of 6e-8 each:
 2e-6), and the features are compute_features' own for that size."""
@@ -16,6 +16,8 @@ def rows_of(kind, n, k, rng):
         p = np.round(rng.random((n, k, 3)) * [3.0, 3.0, 0.6])
     elif kind == "plane":
         p = rng.random((n, k, 3)) * [1.0, 1.0, 0.0]
+    elif kind == "line":
+        p = rng.random((n, k, 1)) * np.array([1.0, 2.0, -0.5])
     elif kind == "duplicates":  # one point, then another one
         p = np.repeat(rng.random((n, 1, 3)), k, 1)
         p[:, 2 * k // 3 :] += 0.25
@@ -40,7 +42,7 @@ def eigentropy64(p, sizes):
 
 
 @pytest.mark.parametrize("n", [3, 700, 6000])
-@pytest.mark.parametrize("kind", ["random", "voxel", "plane", "duplicates", "steady"])
+@pytest.mark.parametrize("kind", ["random", "voxel", "plane", "line", "duplicates", "steady"])
 @pytest.mark.parametrize("k,step", [(20, 1), (73, 1), (74, 1), (110, 1), (110, 7), (75, 64)])
 def test_optimal_size(cuda, pgeof, kind, n, k, step):
     p = rows_of(kind, n, k, np.random.default_rng(k + step))
