@@ -734,6 +734,7 @@ constexpr int kChunkMin = 4;
 constexpr int kGuide = 4;
 constexpr int kSelBins = 64;     // selection histogram
 constexpr int kMaxTries = 6;     // collections of one query before the general kernel takes it
+constexpr float kMinBins = 1e-36f;  // squared radius down to which 1 / it, in bins, is finite
 constexpr int kMaxInBin = 24;    // larger bins (exact ties) fall back to a bitonic sort
 
 struct FastArgs {
@@ -1036,7 +1037,7 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
                     }
                 }
                 if (!ok) {
-                    if (short_knn && optimistic && !guaranteed) {
+                    if (short_knn && optimistic && !guaranteed && tight < 0.0f) {
                         guaranteed = true;
                         continue;
                     }
@@ -1046,7 +1047,8 @@ __device__ __forceinline__ void fast_search_body(const FastArgs& a) {
                     // it with pilot bounds and larger buffers, which took the latency
                     // of the costliest query twice: 0.116 ms on the 1M-point scene,
                     // 0.045 ms on 100k points; this pass pays 0.02-0.03 ms.)
-                    if (!short_knn && attempt + 1 < kMaxTries) {
+                    // Not where the bins' scale overflows (they say nothing then).
+                    if (!short_knn && attempt + 1 < kMaxTries && tau2 >= kMinBins) {
                         const float t = tighter_tau2(ws, k, sb);
                         if (t < tau2) {
                             tight = t;
