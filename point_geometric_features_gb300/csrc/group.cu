@@ -665,8 +665,9 @@ __global__ void __launch_bounds__(32 * kWarps, 6) group_search_kernel(const __gr
                 // one; counted to the end, a few such groups took 1 to 3 million
                 // cycles each and were the kernel's tail (256 scenes: 9.9 -> 7.4
                 // ms; 33 scenes, k = 20: 2.8 -> 1.1 ms; 2 x, 4 x and 8 x alike).
-                // A radius search cannot shrink: it is given up where its 64
-                // parts could not hold it.
+                // A radius search cannot shrink: where its 64 parts could not hold
+                // it, the group is left to the other kernel, as is one whose
+                // rows turn out not to fit a part.
                 const uint32_t give_up = a.stage * (RADIUS ? 64u : 4u);
                 for (int attempt = 0; attempt < 4; ++attempt) {
                     ok = false;
@@ -685,13 +686,14 @@ __global__ void __launch_bounds__(32 * kWarps, 6) group_search_kernel(const __gr
                     n = m.ctl[0];
                     if (n > a.stage) {
                         // too many: a smaller radius, unless that would be short;
-                        // otherwise the rows in several parts
+                        // otherwise the rows in several parts (if all were counted)
                         float less = R * 0.95f * cbrtf((float)a.stage / (float)n);
                         if (!RADIUS && n > give_up) less = fminf(less, a.first * g.h);
                         if (!RADIUS && attempt < 2 && less > too_small * 1.02f) {
                             R = less;
                             continue;
                         }
+                        if (n > give_up) break;
                         parts = (int)min((n + n / 4) / a.stage + 1, 64u);
                     }
                     if (!RADIUS && n < k) {
@@ -704,8 +706,8 @@ __global__ void __launch_bounds__(32 * kWarps, 6) group_search_kernel(const __gr
                     // bins below the last lie wholly inside the R-sphere
                     lim = valid ? kMagic + (uint32_t)(RADIUS ? kBins : kBins - 1) : 0u;
                     bool fits = true;
-                    for (int part = 0; part < parts; ++part) {
-                        if (parts > 1) fits = restage(g, cell_start, a.pts, b, m, a.stage, part, parts, n) && fits;
+                    for (int part = 0; part < parts && fits; ++part) {
+                        if (parts > 1) fits = restage(g, cell_start, a.pts, b, m, a.stage, part, parts, n);
 #pragma unroll 2
                         for (uint32_t c = 4 * w; c < n; c += 4 * kWarps) {
                             const Four f = eval_four(m, c, nx, ny, nz, zero2, sb2);
