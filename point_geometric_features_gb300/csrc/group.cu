@@ -66,6 +66,8 @@ constexpr float kRadiusGap = 1.0f, kRadiusWidth = 6.0f;
 // (1.06 / 1.1: 1.190 / 1.211 ms on the scene, k = 50, 1.196 / 1.211 ms on
 // a uniform cube.)
 constexpr float kGroupSlack = 1.07f;  // R over the largest k-th distance of the group before
+// An SM's shared memory, and what each resident block takes of it besides its own.
+constexpr uint32_t kSmSharedBytes = 228 * 1024, kBlockSharedBytes = 1024;
 constexpr uint32_t kItemGroups = 8;  // groups per work item, at most
 
 // A group of queries: positions [first, first + len) of the sorted queries,
@@ -968,10 +970,8 @@ int launch_group_search(const GroupSearch& q, const SearchOut<float>& out, cudaS
     // k points at `occupancy` points per cell, between a surface's and a volume's
     a.first = powf((float)q.k / (2.0f * q.occupancy), 0.4f);
     a.cap = (q.k + 12 + 1) / 2 * 2;
-    // Room for the candidates of a volume's group (12 k) while it costs no
-    // resident block (1M uniform points, k = 50: 8 k 1.33 ms, 12 k 1.18 ms; scene
-    // k = 100: 8 k 1.34 ms, 12 k 1.61 ms); groups beyond it go in parts. The
-    // turned indices take the same place: 32 rows of tile_width(k) words.
+    // At least so much room for candidates; groups beyond it go in parts. (The turned
+    // indices take the same place: 32 rows of tile_width(k) words.)
     a.stage = (std::max<uint32_t>({256u, (q.k <= 64 ? 12u : 8u) * q.k + 63u, 8 * tile_width(q.k)}) + 31) / 32 * 32;
     a.groups = sp.groups;
     a.group_count = sp.group_count;
@@ -986,9 +986,28 @@ int launch_group_search(const GroupSearch& q, const SearchOut<float>& out, cudaS
     a.rows_sorted = out.rows_in_query_order ? 1 : 0;
     auto kern = rad ? group_search_kernel<MODE_RADIUS, false>
                     : (multi ? group_search_kernel<MODE_KNN, true> : group_search_kernel<MODE_KNN, false>);
-    const int smem = (int)group_smem_bytes(a.k, a.cap, a.stage);
+    int smem = (int)group_smem_bytes(a.k, a.cap, a.stage);
     int per_sm = 0;
     PGEOF_TRY(kernel_blocks_per_sm((const void*)kern, 32 * kWarps, smem, &per_sm));
+    // Then all the shared memory that costs no resident block, but no more than kNN
+    // groups use (a radius search stages whatever its spheres hold). Restaging parts is what
+    // volumes and large radii paid before: 1M uniform points, k = 16 / 24 / 32 1.007 / 0.936 /
+    // 0.974 ms with the minimum, 0.781 / 0.862 / 0.936 with 448 / 608 / 768; half as many
+    // queries as points, k = 16 / 32 / 64 0.976 / 0.932 / 1.076 and 0.683 / 0.777 / 1.003;
+    // radius, 180 found / 10 kept 2.293 and 1.362. The scene, k = 16 / 50: 0.812 / 1.137 and
+    // 0.812 / 1.137. (One block less costs 6 to 12%.)
+    const uint32_t room = kSmSharedBytes / (uint32_t)per_sm - kBlockSharedBytes;
+    if (room > (uint32_t)smem) {
+        const uint32_t most = a.stage + (room - (uint32_t)smem) / 16;
+        const uint32_t want = std::min(rad ? most : std::min(most, 20 * q.k + 192), 2048u) / 32 * 32;
+        const int larger = (int)group_smem_bytes(a.k, a.cap, std::max(a.stage, want));
+        int blocks_then = 0;
+        PGEOF_TRY(kernel_blocks_per_sm((const void*)kern, 32 * kWarps, larger, &blocks_then));
+        if (blocks_then == per_sm) {
+            a.stage = std::max(a.stage, want);
+            smem = larger;
+        }
+    }
     const uint64_t blocks = std::min<uint64_t>(group_cap(q.m), (uint64_t)di->sm_count * per_sm);
     {
         KernelTimer kt("group_search_kernel", s);
