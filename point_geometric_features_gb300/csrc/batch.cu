@@ -332,7 +332,7 @@ int run_pipeline(BatchWorkspace& w, const float* xyz, uint32_t* idx, float* d2, 
     PGEOF_TRY(current_device_info(&di));
     const int nc = w.n_clouds;
     const uint64_t n = w.n;
-    const bool grouped = use_groups(w.n, w.n, w.k);
+    const bool grouped = use_groups(w.n, w.n, w.k, MODE_KNN) != GROUPS_NONE;
     const float target = grouped ? (float)group_occupancy(w.k) * tune.cell
                                  : std::min(48.0f, std::max(2.0f, (float)w.k / 3.5f * tune.cell));
     // 1. bounding boxes

@@ -183,7 +183,7 @@ int knn_impl(const float* data, uint64_t n_data, const float* query, uint64_t n_
              uint32_t* indices, float* sqr_dist, bool query_is_data, cudaStream_t s) {
     if (n_query == 0 || knn == 0) return PGEOF_OK;
     GridIndex<float> grid;
-    PGEOF_TRY(build_grid<float>(data, n_data, knn, 0.0f, 0.0f, grid, s, use_groups(n_data, n_query, knn)));
+    PGEOF_TRY(build_grid<float>(data, n_data, knn, 0.0f, 0.0f, grid, s, use_groups(n_data, n_query, knn, MODE_KNN)));
     SPoint<float>* q = grid.pts;
     const uint32_t* qstart = grid.cell_start;
     Scratch qmem, qstart_mem;
@@ -203,7 +203,7 @@ int radius_impl(const float* data, uint64_t n_data, const float* query, uint64_t
     if (n_query == 0 || max_knn == 0) return PGEOF_OK;
     GridIndex<float> grid;
     const float r = std::fabs(radius);
-    PGEOF_TRY(build_grid<float>(data, n_data, max_knn, r / 4.0f, r, grid, s, use_groups(n_data, n_query, max_knn)));
+    PGEOF_TRY(build_grid<float>(data, n_data, max_knn, r / 4.0f, r, grid, s, use_groups(n_data, n_query, max_knn, MODE_RADIUS)));
     SPoint<float>* q = grid.pts;
     const uint32_t* qstart = grid.cell_start;
     Scratch qmem, qstart_mem;
@@ -839,7 +839,7 @@ int pgeof_knn_features_f32(const float* xyz, int64_t n, uint32_t knn, const uint
     if (n == 0) return PGEOF_OK;
     cudaStream_t s = (cudaStream_t)stream;
     GridIndex<float> grid;
-    PGEOF_TRY(build_grid<float>(xyz, (uint64_t)n, knn, 0.0f, 0.0f, grid, s, use_groups(n, n, knn)));
+    PGEOF_TRY(build_grid<float>(xyz, (uint64_t)n, knn, 0.0f, 0.0f, grid, s, use_groups(n, n, knn, MODE_KNN)));
     // neighbour rows in cell order (no distances): the feature pass then walks
     // spatially adjacent rows, whose neighbourhoods overlap in L1
     Scratch nn, xyz4;

@@ -241,12 +241,17 @@ struct HostBox {
 struct EdgeKey {
     uint64_t n;
     uint32_t k;
-    bool grouped;
+    int groups;
     float h_min, h_max;
     float box[6];
     bool operator==(const EdgeKey& o) const {
-        return n == o.n && k == o.k && grouped == o.grouped && h_min == o.h_min && h_max == o.h_max && memcmp(box, o.box, sizeof(box)) == 0;
+        return n == o.n && k == o.k && groups == o.groups && h_min == o.h_min && h_max == o.h_max &&
+               memcmp(box, o.box, sizeof(box)) == 0;
     }
+};
+struct Edge {
+    double h = 0.0;
+    bool grouped = false, volume = false;
 };
 std::mutex g_edge_mu;
 // 256 entries: a request server cycles through many clouds (the serving
@@ -254,28 +259,28 @@ std::mutex g_edge_mu;
 // host round trips.
 constexpr int kEdgeCache = 256;
 EdgeKey g_edge_keys[kEdgeCache];
-double g_edge_vals[kEdgeCache];
+Edge g_edge_vals[kEdgeCache];
 int g_edge_n = 0, g_edge_next = 0;
 
-bool edge_cache_get(const EdgeKey& k, double& h) {
+bool edge_cache_get(const EdgeKey& k, Edge& e) {
     std::lock_guard<std::mutex> lk(g_edge_mu);
     for (int i = 0; i < g_edge_n; ++i)
         if (g_edge_keys[i] == k) {
-            h = g_edge_vals[i];
+            e = g_edge_vals[i];
             return true;
         }
     return false;
 }
 
-void edge_cache_put(const EdgeKey& k, double h) {
+void edge_cache_put(const EdgeKey& k, const Edge& e) {
     std::lock_guard<std::mutex> lk(g_edge_mu);
     for (int i = 0; i < g_edge_n; ++i)
         if (g_edge_keys[i] == k) {
-            g_edge_vals[i] = h;
+            g_edge_vals[i] = e;
             return;
         }
     g_edge_keys[g_edge_next] = k;
-    g_edge_vals[g_edge_next] = h;
+    g_edge_vals[g_edge_next] = e;
     g_edge_next = (g_edge_next + 1) % kEdgeCache;
     g_edge_n = std::min(g_edge_n + 1, kEdgeCache);
 }
@@ -353,7 +358,7 @@ int exclusive_scan_into(const uint32_t* in, uint32_t G, uint32_t* out, uint32_t*
 
 template <typename T>
 int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h_max, GridIndex<T>& out,
-               cudaStream_t s, bool grouped) {
+               cudaStream_t s, int groups) {
     out.n = n;
     if (n == 0) return PGEOF_OK;
     if (n >= 0xffffffffull) return fail(PGEOF_ERR_INVALID_ARGUMENT, "point clouds are limited to 2^32-1 points");
@@ -398,8 +403,10 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
     // k / 12 is 19% faster at k = 50 than k / 3.5, on an outdoor scene of
     // walls and ground k / 3.5 is best. The dimension comes from two trial
     // histograms: (occupancy - 1) scales as h^dim (the 1 is the point itself).
-    out.grouped = grouped ? (float)group_occupancy(k_target) : 0.0f;
-    const double target2 = grouped ? group_occupancy(k_target) : std::min(48.0, std::max(2.0, (double)k_target / 3.5));
+    Edge edge;
+    edge.grouped = groups != GROUPS_NONE;
+    const double target2 =
+        edge.grouped ? group_occupancy(k_target) : std::min(48.0, std::max(2.0, (double)k_target / 3.5));
     const uint64_t cap = std::max<uint64_t>(4 * n, 1u << 16);
     const double hmin = h_min > 0 ? (double)h_min : 0.0;
     const double hmax = h_max > 0 ? (double)h_max : 1e300;
@@ -413,10 +420,9 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
     };
     double h0 = clamp_h(std::cbrt(vol * target2 / (double)n));
     double h = h0;
-    EdgeKey key{n, k_target, grouped, h_min, h_max, {b.mn[0], b.mn[1], b.mn[2], b.mx[0], b.mx[1], b.mx[2]}};
-    double cached = 0.0;
-    if (edge_cache_get(key, cached)) {
-        h = cached;
+    EdgeKey key{n, k_target, groups, h_min, h_max, {b.mn[0], b.mn[1], b.mn[2], b.mx[0], b.mx[1], b.mx[2]}};
+    if (edge_cache_get(key, edge)) {
+        h = edge.h;
     } else if (n > 64) {
         GridParams g;
         make_params(b, h0, cap, g);
@@ -440,29 +446,43 @@ int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h
                     h = clamp_h(h1 * std::pow(target2 / m1, 1.0 / dim));
                 }
             }
-        } else if (m0 > 0.0) {
-            // on target at the first trial: a half-edge trial for the dimension
+        }
+        if (h1 == h0 && m0 > 0.0 && (groups != GROUPS_NONE || (m0 > target2 / 1.6 && m0 < target2 * 1.6))) {
+            // on target at the first trial, or held by the radius: a half-edge trial for
+            // the dimension
             h1 = clamp_h(h0 * 0.5);
             if (h1 != h0) {
                 make_params(b, h1, cap, g);
                 PGEOF_TRY(occupancy<T>(xyz, n, g, cnt.as<uint32_t>(), acc, m1, s));
             }
         }
-        // volume-filling clouds: finer cells, placed by (m - 1) ~ h^dim
-        if (!grouped && m0 > 1.05 && m1 > 1.05 && h1 != h0) {
-            double dim = std::log((m0 - 1.0) / (m1 - 1.0)) / std::log(h0 / h1);
+        // (m - 1) ~ h^dim, from the two trials
+        const bool fitted = m0 > 1.05 && m1 > 1.05 && h1 != h0;
+        double dim = 2.0;
+        if (fitted) {
+            dim = std::log((m0 - 1.0) / (m1 - 1.0)) / std::log(h0 / h1);
             if (!std::isfinite(dim)) dim = 2.0;
             dim = std::min(3.0, std::max(1.0, dim));
-            const double w = std::min(1.0, std::max(0.0, (dim - 2.3) / 0.6));
-            if (w > 0.0) {
-                const double target = std::min(48.0, std::max(2.0, (double)k_target / (3.5 + 8.5 * w)));
-                const bool use1 = std::fabs(std::log(m1 / target)) < std::fabs(std::log(m0 / target));
-                const double hr = use1 ? h1 : h0, mr = use1 ? m1 : m0;
-                h = clamp_h(hr * std::pow((target - 1.0) / (mr - 1.0), 1.0 / dim));
-            }
+        }
+        const double w = std::min(1.0, std::max(0.0, (dim - 2.3) / 0.6));
+        edge.volume = w > 0.5;
+        if (edge.grouped && h_max > 0) {
+            const double m = h == h0 || !(m1 > 0.0) ? m0 : m1 + (m1 - 1.0) * (std::pow(h / h1, dim) - 1.0);
+            if (!radius_groups_fill(m, edge.volume, k_target)) edge.grouped = false;
+        }
+        if (edge.volume && groups == GROUPS_SURFACES) edge.grouped = false;
+        // volume-filling clouds: finer cells
+        if (!edge.grouped && fitted && w > 0.0) {
+            const double target = std::min(48.0, std::max(2.0, (double)k_target / (3.5 + 8.5 * w)));
+            const bool use1 = std::fabs(std::log(m1 / target)) < std::fabs(std::log(m0 / target));
+            const double hr = use1 ? h1 : h0, mr = use1 ? m1 : m0;
+            h = clamp_h(hr * std::pow((target - 1.0) / (mr - 1.0), 1.0 / dim));
         }
     }
-    edge_cache_put(key, h);
+    edge.h = h;
+    edge_cache_put(key, edge);
+    out.grouped = edge.grouped ? (float)group_occupancy(k_target) : 0.0f;
+    out.volume = edge.volume;
     // the final grid splits cells along x (see GridParams) while the cell
     // table stays within 8 entries per point
     GridParams g;
@@ -533,8 +553,8 @@ int sort_queries(const T* q, uint64_t m, const GridParams& g, Scratch& out_mem, 
     return check_launch("scatter_kernel(queries)");
 }
 
-template int build_grid<float>(const float*, uint64_t, uint32_t, float, float, GridIndex<float>&, cudaStream_t, bool);
-template int build_grid<double>(const double*, uint64_t, uint32_t, float, float, GridIndex<double>&, cudaStream_t, bool);
+template int build_grid<float>(const float*, uint64_t, uint32_t, float, float, GridIndex<float>&, cudaStream_t, int);
+template int build_grid<double>(const double*, uint64_t, uint32_t, float, float, GridIndex<double>&, cudaStream_t, int);
 template int sort_queries<float>(const float*, uint64_t, const GridParams&, Scratch&, SPoint<float>**, Scratch&,
                                  cudaStream_t);
 template int sort_queries<double>(const double*, uint64_t, const GridParams&, Scratch&, SPoint<double>**, Scratch&,

@@ -62,7 +62,7 @@ constexpr float kGroupWidth = 2.0f;
 // 0.56 / 64: one query per warp 2.35 ms, gap / width 0.75 / 2 2.42, 1 / 4 2.19, 1 / 6
 // 2.18, 1.5 / 8 2.16; 400k points, 0.4 / 30: 0.41, 0.46, 0.40, 0.39, 0.38; dense
 // clouds cut their runs at 32 members first: 4M points, 0.5 / 64 4.39, 4.40, 4.40, 4.41).
-constexpr float kRadiusGap = 1.0f, kRadiusWidth = 6.0f;
+constexpr float kRadiusGap = 1.0f;
 // (1.06 / 1.1: 1.190 / 1.211 ms on the scene, k = 50, 1.196 / 1.211 ms on
 // a uniform cube.)
 constexpr float kGroupSlack = 1.07f;  // R over the largest k-th distance of the group before

@@ -11,6 +11,7 @@
 // and any stream of the same device may search it concurrently. Every search
 // records an event on its stream; pgeof_index_destroy makes the index's own
 // stream wait for those events before the memory goes back to the pool.
+#include <algorithm>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -131,10 +132,14 @@ int pgeof_index_create_f32(const float* data, int64_t n_data, uint32_t k_hint, f
     int st = PGEOF_OK;
     if (cudaGetDevice(&ix->device) != cudaSuccess) st = fail(PGEOF_ERR_CUDA, "cudaGetDevice");
     // the cell-size rule of the per-call entry points: kNN steers the occupancy
-    // towards k, a radius clamps the edge to [r/4, r]
+    // towards k, a radius clamps the edge to [r/4, r]. Cells for groups on surfaces only:
+    // there they serve small query sets as well as the others do, or better (1M-point scene,
+    // k = 16, 1k / 100k queries / all: 126 -> 99 / 275 -> 227 / 1069 -> 733 us), while in a
+    // volume queries that do not go by groups want the finer cells (uniform points, k = 50,
+    // 100k / 400k queries / all: 260 and 344 / 670 and 894 / 1285 and 1106 us).
     if (st == PGEOF_OK)
         st = build_grid<float>(data, ix->n, ix->k_hint, radius_hint / 4.0f, radius_hint, ix->grid, s,
-                               use_groups(ix->n, ix->n, ix->k_hint));
+                               std::min(GROUPS_SURFACES, use_groups(ix->n, ix->n, ix->k_hint, MODE_KNN)));
     if (st == PGEOF_OK) st = ix->xyz4.alloc(ix->n * sizeof(float4), s);
     if (st == PGEOF_OK) {
         const int blocks = (int)std::min<uint64_t>((ix->n + 255) / 256, 4096);

@@ -111,15 +111,16 @@ struct GridIndex {
     SPoint<T>* pts = nullptr;        // n (device), cell order
     Scratch cell_mem, pts_mem;
     float grouped = 0.0f;  // > 0: cells sized for the grouped search, with this occupancy
+    bool volume = false;   // the points fill a volume rather than lie on surfaces
 };
 
 // Build the index of `xyz` (device, row-major (n, 3)). `k_target` steers the
 // cell size towards ~k_target/3.5 points per cell around an average point;
-// `h_min`/`h_max` (> 0) clamp the edge (radius searches). `grouped`: cells for
-// the grouped search.
+// `h_min`/`h_max` (> 0) clamp the edge (radius searches). `groups` (enum Groups,
+// group.cuh): on which clouds the cells are for the grouped search.
 template <typename T>
 int build_grid(const T* xyz, uint64_t n, uint32_t k_target, float h_min, float h_max, GridIndex<T>& out,
-               cudaStream_t s, bool grouped = false);
+               cudaStream_t s, int groups = 0);
 
 // Counting-sort arbitrary query points into `grid`'s cell order; `start`
 // receives the per-cell offsets of the sorted queries (n_cells + 1).

@@ -1335,7 +1335,8 @@ int launch_search(const GridIndex<T>& grid, const SPoint<T>* queries, const uint
         if (k > 128 || m >= 0xfff00000ull)  // 32-bit work counters with headroom for the last items
             return launch_general<T>(grid, queries, m, nullptr, nullptr, mode, k, radius, out, s);
         Scratch ctl;
-        const float occupancy = use_groups(grid.n, m, k) ? grid.grouped : 0.0f;
+        const Groups groups = use_groups(grid.n, m, k, mode);
+        const float occupancy = groups == GROUPS_ALL || (groups == GROUPS_SURFACES && !grid.volume) ? grid.grouped : 0.0f;
         const uint64_t block_words = occupancy > 0.0f && m >= kOrderMin ? group_block_words(grid.g) : 0;
         PGEOF_TRY(ctl.alloc(fast_words(m, block_words) * sizeof(uint32_t), s));
         GridView<float> gv;
