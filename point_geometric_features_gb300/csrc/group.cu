@@ -252,7 +252,7 @@ __device__ __forceinline__ void take_four(const uint32_t (&bits)[4], const uint3
 // The block's shared memory.
 struct Smem {
     uint32_t* hist;   // [kBins][32] counts, then cursors; later the turned d^2, [32][T]
-    uint32_t* keys;   // [cap][2][32]: d^2 bits, index; a row before (-1) and a row after (kEmptyKey)
+    uint32_t* keys;   // [cap][2][32]: d^2 bits, index; and a row after (kEmptyKey)
     float* x;         // staged candidates, [stage] each; later the turned indices, [32][T]
     float* y;
     float* z;
@@ -267,12 +267,12 @@ __host__ __device__ inline uint32_t hist_words(uint32_t k) {
     return kBins * 32 > 32 * tile_width(k) ? kBins * 32 : 32 * tile_width(k);
 }
 __host__ __device__ inline size_t group_smem_bytes(uint32_t k, uint32_t cap, uint32_t stage) {
-    return 4 * ((size_t)hist_words(k) + 64 * ((size_t)cap + 2) + 4 * (size_t)stage + 32 * kWarps + 64 + 8);
+    return 4 * ((size_t)hist_words(k) + 64 * ((size_t)cap + 1) + 4 * (size_t)stage + 32 * kWarps + 64 + 8);
 }
 __device__ __forceinline__ Smem carve(uint32_t* base, uint32_t k, uint32_t cap, uint32_t stage) {
     Smem m;
     m.hist = base;
-    m.keys = m.hist + hist_words(k) + 64;
+    m.keys = m.hist + hist_words(k);
     m.x = reinterpret_cast<float*>(m.keys + 64 * (cap + 1));
     m.y = m.x + stage;
     m.z = m.y + stage;
@@ -371,10 +371,9 @@ __device__ __forceinline__ Four eval_four(const Smem& m, uint32_t c, unsigned lo
 // ranks in the turned tiles. The column is sorted by bins of at most `widest`
 // keys, so a key is out of place by less than that: its rank is its row, plus
 // the smaller keys among the next widest - 1 rows, minus the larger ones among
-// the last widest - 1. Rows outside the column hold smaller (negative) and
-// larger (kEmptyKey) values than any key; as signed integers d^2 bits keep
-// their order. Keys that tie keep the order of their rows (see the rows' way
-// out).
+// the last widest - 1; each of those rows is read once for all four. Rows behind the
+// column hold larger values (kEmptyKey) than any key; as signed integers d^2 bits
+// keep their order. Keys that tie keep the order of their rows (order_ties).
 struct Turn {
     uint32_t* tile_d;
     uint32_t* tile_i;
@@ -384,49 +383,31 @@ struct Turn {
 constexpr int kRankRows = 4;
 __device__ __forceinline__ void rank_rows(const uint32_t* col, int j0, int n, int cap, int widest, const Turn& turn) {
     int d[kRankRows], r[kRankRows];
-    if (j0 - widest >= -1 && j0 + kRankRows - 1 + widest <= cap) {
-        // two rows further to either side at a time, from a window in registers
-        const uint32_t* up = col + 64 * j0;
-        const uint32_t* down = up;
-        int u[kRankRows + 2], v[kRankRows + 2];
 #pragma unroll
-        for (int t = 0; t < kRankRows; ++t) {
-            d[t] = u[t] = v[t] = (int)up[64 * t];
-            r[t] = j0 + t;
+    for (int t = 0; t < kRankRows; ++t) {
+        d[t] = (int)col[64 * min(j0 + t, cap)];
+        r[t] = j0 + t;
+    }
+#pragma unroll
+    for (int t = 0; t < kRankRows; ++t)
+#pragma unroll
+        for (int o = t + 1; o < kRankRows; ++o) {
+            const int swap = d[o] < d[t];
+            r[t] += swap;
+            r[o] -= swap;
         }
-        for (int o = 1; o < widest; o += 2) {
-            u[kRankRows] = (int)up[64 * kRankRows];
-            u[kRankRows + 1] = (int)up[64 * (kRankRows + 1)];
-            const int w0 = (int)down[-64], w1 = (int)down[-128];  // rows before the window
-            up += 128;
-            down -= 128;
+    const int first = max(j0 - widest + 1, 0), last = min(j0 + kRankRows + widest - 2, cap);
+#pragma unroll 2
+    for (int o = j0 - 1; o >= first; --o) {
+        const int e = (int)col[64 * o];
 #pragma unroll
-            for (int t = 0; t < kRankRows; ++t) {
-                r[t] += u[t + 1] < d[t];
-                r[t] += u[t + 2] < d[t];
-                r[t] -= (t >= 1 ? v[t - 1] : w0) > d[t];
-                r[t] -= (t >= 2 ? v[t - 2] : (t == 1 ? w0 : w1)) > d[t];
-            }
+        for (int t = 0; t < kRankRows; ++t) r[t] -= e > d[t];
+    }
+#pragma unroll 2
+    for (int o = j0 + kRankRows; o <= last; ++o) {
+        const int e = (int)col[64 * o];
 #pragma unroll
-            for (int t = 0; t < kRankRows; ++t) u[t] = u[t + 2];
-#pragma unroll
-            for (int t = kRankRows - 1; t >= 2; --t) v[t] = v[t - 2];
-            v[1] = w0;
-            v[0] = w1;
-        }
-    } else {
-#pragma unroll
-        for (int t = 0; t < kRankRows; ++t) {
-            d[t] = (int)col[64 * min(j0 + t, cap)];
-            r[t] = j0 + t;
-        }
-#pragma unroll 1
-        for (int o = 1; o < widest; ++o)
-#pragma unroll
-            for (int t = 0; t < kRankRows; ++t) {
-                r[t] += (int)col[64 * min(j0 + t + o, cap)] < d[t];
-                r[t] -= (int)col[64 * max(j0 + t - o, -1)] > d[t];
-            }
+        for (int t = 0; t < kRankRows; ++t) r[t] += e < d[t];
     }
 #pragma unroll
     for (int t = 0; t < kRankRows; ++t)
@@ -436,18 +417,59 @@ __device__ __forceinline__ void rank_rows(const uint32_t* col, int j0, int n, in
         }
 }
 
-// A row in which distances tie: its first `have` keys by (d^2, index), each by
-// its rank among all n keys of the query's column. (Warp-wide call.)
-template <typename Put>
-__device__ __noinline__ void tied_row(const uint32_t* col, int n, int have, Put put) {
-    for (int j = threadIdx.x & 31; j < n; j += 32) {
-        const uint32_t d = col[64 * j], i = col[64 * j + 32];
-        int r = 0;
-        for (int t = 0; t < n; ++t) {
-            const uint32_t e = col[64 * t];
-            r += e < d || (e == d && col[64 * t + 32] < i);
+// Puts the indices of a row in which distances tie in their order: among equal
+// distances the smaller index comes first. td / ti: the row's keys by distance, `have`
+// of them, and one more if the column has (all > have); col: the column, whose last
+// `widest` keys hold the k-th distance's bin; out: the row, written by distance already.
+// A run of equal distances sorts itself by counting, passed from lane to lane. One that
+// the row's end cuts through takes its indices from the column. (Warp-wide call. Every key
+// against all of the column took as long as a row's search: a million points on a 5 cm
+// grid, k = 32 / 50: 1.64 / 2.59 ms, now 1.06 / 1.35; without ties 0.94 / 1.14.)
+__device__ __noinline__ void order_ties(const uint32_t* td, const uint32_t* ti, const uint32_t* col, int have, int all,
+                                        int widest, uint32_t* out) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t dk = td[have - 1];
+    const bool cut = have < all && td[have] == dk;
+    int before = 0;  // the lane's keys nearer than dk
+    for (int base = 0; base < have; base += 32) {
+        const int j = base + lane;
+        const uint32_t d = j < have ? td[j] : 0xffffffffu, i = ti[min(j, have - 1)];
+        const bool in = j < have && !(cut && d == dk);
+        before += in;
+        const uint32_t left = __shfl_up_sync(FULL, d, 1);
+        const uint32_t heads = ~__ballot_sync(FULL, lane > 0 && left == d);  // of runs of one distance
+        const int start = 31 - __clz(heads & (FULL >> (31 - lane)));
+        const uint32_t after = lane == 31 ? 0u : heads & (FULL << (lane + 1));
+        const int stop = after ? __ffs(after) - 1 : 32;
+        const int longest = __reduce_max_sync(FULL, in ? stop - start : 0);
+        int r = j;
+        for (int o = 1; o < longest; ++o) {
+            const uint32_t up = __shfl_up_sync(FULL, i, o), down = __shfl_down_sync(FULL, i, o);
+            if (lane - o >= start) r -= up > i;
+            if (lane + o < stop) r += down < i;
         }
-        if (r < have) put(r, i, d);
+        // runs that reach beyond these 32
+        if (in && start == 0)
+            for (int o = base - 1; o >= 0 && td[o] == d; --o) r -= ti[o] > i;
+        if (in && stop == 32)
+            for (int o = base + 32; o < have && td[o] == d; ++o) r += ti[o] < i;
+        if (in && r != j) out[r] = i;
+    }
+    __syncwarp();
+    if (!cut) return;
+    before = __reduce_add_sync(FULL, before);
+    const int lo = max(0, all - widest);
+    for (int base = lo; base < all; base += 32) {
+        const int t = base + lane;
+        const bool mine = t < all && col[64 * min(t, all - 1)] == dk;
+        const uint32_t i = col[64 * min(t, all - 1) + 32];
+        int r = before;
+        if (all - lo <= 32) {
+            for (uint32_t left = __ballot_sync(FULL, mine); left; left &= left - 1) r += __shfl_sync(FULL, i, __ffs(left) - 1) < i;
+        } else {
+            for (int o = lo; o < all; ++o) r += col[64 * o] == dk && col[64 * o + 32] < i;
+        }
+        if (mine && r < have) out[r] = i;
     }
 }
 
@@ -614,7 +636,6 @@ __global__ void __launch_bounds__(32 * kWarps, 6) group_search_kernel(const __gr
     const uint32_t hbase = (uint32_t)__cvta_generic_to_shared(m.hist) + 4u * lane - (kMagic << 7);
     const uint32_t k = a.k, T = tile_width(a.k);
     const uint32_t n_groups = *a.group_count;
-    if (w == 0) (m.keys - 64)[lane] = 0xffffffffu;  // the row before every column
     const unsigned long long zero2 = a.zero2;
     for (;;) {
         __syncthreads();
@@ -829,12 +850,9 @@ __global__ void __launch_bounds__(32 * kWarps, 6) group_search_kernel(const __gr
                             if (a.out_d2) *reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(o) + to_d2) = d;
                         }
                         if (__any_sync(FULL, tie)) {
-                            uint32_t* row0 = reinterpret_cast<uint32_t*>(__shfl_sync(FULL, first, q));
-                            __syncwarp();
-                            tied_row(m.keys + q, (int)all, (int)have, [&](int r, uint32_t i, uint32_t d) {
-                                row0[r] = i;
-                                if (a.out_d2) *reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(row0 + r) + to_d2) = d;
-                            });
+                            __syncwarp();  // (the row as written above)
+                            order_ties(td, ti, m.keys + q, (int)have, (int)all, widest,
+                                       reinterpret_cast<uint32_t*>(__shfl_sync(FULL, first, q)));
                         }
                     }
                     if (RADIUS && a.out_found && ok && w == 0) a.out_found[row] = found;
