@@ -770,12 +770,12 @@ constexpr float kTieBand = 3e-5f;
 // reference covariance. Rows that need an exact solve (near-tied sizes, 0.4% of
 // a scene's; small eigen-gaps) are queued for optimal_exact_kernel.
 //
-// What bounds it: instruction issue (68% of slots), after the gathers' latency
+// What bounds it: instruction issue (72% of slots, 23 of 32 threads), after the gathers' latency
 // and L1 look-ups in the scan (one random 16-byte read per neighbour). So four
 // points are in flight per thread while four are handled, indices come four at
 // a time, moments are summed in packed pairs, and only near-tied sizes are kept
 // (one eigentropy per size took 32 KB of shared memory a block and half the
-// resident warps). 4M rows of up to 64 neighbours: 5.98 -> 3.16 ms, and 0.22 ms
+// resident warps). 4M rows of up to 64 neighbours: 5.98 -> 3.18 ms, and 0.15 ms
 // for the queue. Blocks of 64 x 12 / 128 x 6 / 128 x 5 / 32 x 20 per SM: 3.16 /
 // 3.20 / 3.29 / 3.22 ms.
 __global__ void __launch_bounds__(kOptThreads, 12) optimal_kernel(const __grid_constant__ OptArgs a) {
